@@ -310,6 +310,12 @@ inline void put_digit(uint8_t* row, bool nib, int kb, int e, uint32_t d) {
     }
 }
 
+// Right shift from the fixed point of a component (exponent beta) to that of a
+// row tile (c_exp >= beta); 63 stands for "nothing left".
+int32_t fixed_shift(int32_t c_exp, int32_t beta) {
+    return beta == kNoExp ? 63 : std::min<int32_t>(63, c_exp - beta);
+}
+
 // Longest run of chunks one column unit walks: kMaxPartChunks, or fewer when
 // the environment variable QHMAT_GB300_PART_CHUNKS (1 .. kMaxPartChunks) asks
 // for it -- a test knob that sends short tasks through the split-task path
@@ -390,7 +396,6 @@ Layout build_layout(const HostMatrix& m) {
                      [](const auto& a, const auto& b) { return a.first < b.first; });
     std::vector<ColTask> tasks;
     std::vector<TaskRec> task_rec;
-    std::vector<int32_t> comp_part(m.width.size(), -1);  // row of a split task's partial sums, or -1
     std::vector<uint8_t> qcodes;
     int32_t n_split = 0;
     for (size_t i = 0; i < comps.size();) {
@@ -407,9 +412,7 @@ Layout build_layout(const HostMatrix& m) {
             const int32_t comp_idx = int32_t(task_rec.size());
             for (int32_t l = 0; l < count; ++l) {
                 const int32_t c = comps[t0 + l].second;
-                // One rounding: s_P * s_Q.  In exact arithmetic the block contribution
-                // sum_j (s_P c_P)(sum_k s_Q c_Q x) equals sum_j c_P (s_P s_Q) sum_k c_Q x.
-                task_rec.push_back({c, key.w, m.left_scale[size_t(c)] * m.right_scale[size_t(c)]});
+                task_rec.push_back({c, uint8_t(key.w), 1, 0, 0});
             }
             const size_t base = qcodes.size();  // multiple of 16 bytes
             qcodes.resize(base + size_t(nchunks) * size_t(stride), 0);
@@ -438,13 +441,19 @@ Layout build_layout(const HostMatrix& m) {
                         goff += size_t(rows_q) * rb;
                     }
                 }
-                const double bound = l1 * std::fabs(m.left_scale[size_t(c)] * m.right_scale[size_t(c)]);
-                if (bound > 0.0 && std::isfinite(bound)) beta[size_t(c)] = int32_t(std::ilogb(bound)) + 2;
+                // One rounding: s_P * s_Q.  In exact arithmetic the block contribution
+                // sum_j (s_P c_P)(sum_k s_Q c_Q x) equals sum_j c_P (s_P s_Q) sum_k c_Q x.
+                const double s = m.left_scale[size_t(c)] * m.right_scale[size_t(c)];
+                const double bound = l1 * std::fabs(s);
+                if (bound > 0.0 && std::isfinite(bound)) {
+                    beta[size_t(c)] = int32_t(std::ilogb(bound)) + 2;
+                    TaskRec& R = task_rec[size_t(comp_idx + l)];
+                    R.shift = uint8_t(std::ilogb(l1) + 1);
+                    R.kappa = uint64_t(std::ldexp(s, 64 + int(R.shift) - beta[size_t(c)]));
+                }
             }
             const int32_t nparts = (nchunks + part_chunks - 1) / part_chunks;
             const int32_t split_id = nparts > 1 ? n_split++ : -1;
-            if (split_id >= 0)
-                for (int32_t l = 0; l < count; ++l) comp_part[size_t(comps[t0 + l].second)] = split_id * 33 + l;
             L.max_parts = std::max(L.max_parts, nparts);
             const int32_t cps = std::max<int32_t>(1, kColSlotBytes / (stride + kColChunk * 16));
             for (int32_t pt = 0; pt < nparts; ++pt) {
@@ -496,7 +505,7 @@ Layout build_layout(const HostMatrix& m) {
     std::vector<uint8_t> kp_info;
     int64_t n_slots = 0;
     std::vector<TileDense> tdense;
-    std::vector<SlotRec> slot_rec;   // each B row slot's component, split row and width
+    std::vector<SlotRec> slot_rec;   // each B row slot's component, shift and width
     std::vector<std::vector<std::pair<int32_t, int32_t>>> comp_dest(m.width.size());  // per component: (slot, tile)
     std::vector<uint32_t> row_steps; // pipeline steps of the row units
     struct RowComp {
@@ -556,7 +565,7 @@ Layout build_layout(const HostMatrix& m) {
                         const int32_t k = 32 * kp + e;
                         if (k < K) {
                             const int32_t c = kc[size_t(k)].comp;
-                            slot_rec.push_back({c, ((comp_part[size_t(c)] + 1) << 8) | int32_t(m.width[size_t(c)])});
+                            slot_rec.push_back({c, (fixed_shift(T.c_exp, beta[size_t(c)]) << 8) | int32_t(m.width[size_t(c)])});
                             comp_dest[size_t(c)].push_back({int32_t(slot_rec.size() - 1), ti});
                         } else {
                             slot_rec.push_back({-1, 1});
@@ -657,8 +666,8 @@ Layout build_layout(const HostMatrix& m) {
             std::vector<std::pair<int32_t, TaskDest>> lst;  // (tile, record)
             for (int32_t r = 0; r < T.count; ++r)
                 for (const auto& [slot, ti] : comp_dest[size_t(task_rec[size_t(T.comp_idx + r)].comp)]) {
-                    const int32_t ce = tiles[size_t(ti)].c_exp;
-                    lst.push_back({ti, {slot, (r << 16) | int32_t(uint16_t(int16_t(ce)))}});
+                    const int32_t c = task_rec[size_t(T.comp_idx + r)].comp;
+                    lst.push_back({ti, {slot, (r << 16) | fixed_shift(tiles[size_t(ti)].c_exp, beta[size_t(c)])}});
                 }
             std::stable_sort(lst.begin(), lst.end(), [](const auto& a, const auto& b) { return a.first < b.first; });
             for (const auto& e : lst) task_dest.push_back(e.second);

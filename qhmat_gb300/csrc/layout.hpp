@@ -135,18 +135,29 @@ struct ColTask {
     int32_t dest0, ndest;
 };
 // A row-side B row fed by a column task: slot, and (component row in the
-// task) << 16 | the tile's exponent offset as a 16-bit signed field.  A task's
-// list is ordered by (tile, row), so that a tile's B rows are consecutive.
+// task) << 16 | the right shift (0 .. 63) from the component's fixed point to
+// the tile's.  A task's list is ordered by (tile, row), so that a tile's B
+// rows are consecutive.
 struct TaskDest {
     int32_t slot, row_cexp;
 };
 static_assert(sizeof(TaskDest) == 8, "TaskDest layout");
 static_assert(sizeof(ColTask) == 64, "ColTask layout");
 // Finalize operands of one component of a column task (one 16-byte load).
+// The component's u = s t 2^(xe - 1022 - kFixBits), s = s^P s^Q, t its exact
+// integer sum, is held in fixed point on the component's own exponent,
+// V = round(u 2^(kFixBits - (xe - 1022 + beta))) = round(t s 2^-beta), beta a
+// layout-time bound (|u| < 2^(xe - 1022 + beta), so |V| < 2^kFixBits).  With
+// 2^(shift - 1) <= sum |c| < 2^shift, t 2^-shift fits 63 bits and
+// s 2^(shift - beta) lies in [1/4, 1): kappa is that factor times 2^64
+// (exact, the product s having 53 bits), and V = (t >> shift) kappa >> 64.
 struct TaskRec {
-    int32_t comp, width;
-    double scale;  // s^P s^Q
+    int32_t comp;
+    uint8_t width, shift;
+    uint16_t pad;
+    uint64_t kappa;  // 0: u is identically zero
 };
+static_assert(sizeof(TaskRec) == 16, "TaskRec layout");
 struct DenseDesc {
     int32_t row0, m, col0, n;
     int64_t off;  // element offset of the column-major values in the dense arena
@@ -185,8 +196,8 @@ struct RowUnit {
 static_assert(sizeof(RowUnit) == 64, "RowUnit layout");
 
 // A row-side B row slot: its component (-1: padding past the tile's k axis)
-// and (split row + 1) << 8 | width (split row: the component's row in the
-// partial sums of a split column task, as split_id * 33 + row; 0: unsplit).
+// and shift << 8 | width (shift: from the component's fixed point to the
+// tile's, as in TaskDest).
 struct SlotRec {
     int32_t comp, info;
 };

@@ -10,16 +10,18 @@
 // FP64 throughput on GB300 is a small fraction of its tensor throughput, so
 // every code product is an exact small-integer product on the f16 tensor
 // cores (digits <= 255 times 8-bit limbs of a fixed-point operand, FP32 sums
-// that stay integers below 2^24), and FP64 is used only per component, per
-// output row and for the dense diagonal blocks:
+// that stay integers below 2^24), and FP64 is used only per output row and for
+// the dense diagonal blocks:
 //
 //   prep_x / x_limbs   x (source order) -> clustered order; one exponent per
 //                      rhs column; X = round(x 2^(62-e)) as eight f16 limbs.
 //   column_kernel      warp per task (<= 32 components sharing a column range
 //                      and a width): t_j = sum_i c_ij X_i exactly, then
-//                      u_j = (s^P s^Q) t_j 2^(e-1022-62) in FP64, then u in
-//                      fixed point on each consuming row tile's exponent (a
-//                      layout-time bound) as that tile's B rows (limbs);
+//                      u_j = (s^P s^Q) t_j 2^(e-1022-62) in fixed point on the
+//                      component's own exponent (a layout-time bound; one
+//                      64 x 64-bit integer product), then shifted to each
+//                      consuming row tile's exponent as that tile's B rows
+//                      (limbs);
 //                      and warp per dense unit (16 columns of a dense
 //                      diagonal block part, FP64 row sums).
 //   row_kernel         warp per (row tile, 16 rows, k split): sum_j c_ij U_j
@@ -28,8 +30,9 @@
 //                      the partials -> y (one conversion).
 //
 // The only rounding steps are the fixed-point conversions of x and u (2^-63
-// of the column's largest |x|, of the tile's bound on |u|), the product
-// s^P s^Q, and the final FP64 conversions: the result agrees with the
+// of the column's largest |x|, ~2^-62 of the component's and of the tile's
+// bound on |u|), the product s^P s^Q, and the final FP64 conversions: the
+// result agrees with the
 // reference's FP64 matmul (src/qhmat/core.cpp:360-390) to ~1e-15 in norm.
 #include <cooperative_groups.h>
 #include <cuda_fp16.h>
@@ -53,156 +56,10 @@
 #include "batch.hpp"
 #include "errors.hpp"
 #include "layout.hpp"
+#include "plain.hpp"
 
 namespace qhg {
 namespace {
-
-// Fixed point: x (per rhs column) and u (per row tile) are held as integers
-// X = round(v * 2^(kFixBits - (e - 1022))), |X| <= 2^kFixBits, on one exponent
-// field e; the tensor-core operand is X's eight base-256 limbs (seven unsigned,
-// the top one signed), each an exact f16.
-constexpr int kFixBits = 62;
-
-
-// ---------------------------------------------------------------- helpers
-
-// Biased IEEE exponent field; 0 for zero/subnormal.  |v| < 2^(e - 1022).
-__device__ __forceinline__ int exp_field(double v) {
-    return int((__double_as_longlong(v) >> 52) & 0x7FF);
-}
-
-// round(v * 2^(kFixBits - (emax - 1022))) as an integer, computed with integer
-// operations only (the FP64 pipe is the scarce one).  emax must be >= the
-// exponent field of v; subnormals give 0.
-__device__ __forceinline__ long long to_fixed(double v, int emax) {
-    const long long bits = __double_as_longlong(v);
-    const int e = int((bits >> 52) & 0x7FF);
-    if (e == 0) return 0;
-    const long long mant = (bits & 0xFFFFFFFFFFFFFLL) | 0x10000000000000LL;
-    const int rs = emax - e + (1075 - 1022 - kFixBits);  // right shift, >= 53 - kFixBits
-    long long q;
-    if (rs <= 0) q = mant << (-rs);
-    else q = rs >= 62 ? 0 : ((mant + (1LL << (rs - 1))) >> rs);
-    return bits < 0 ? -q : q;
-}
-
-__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
-    uint32_t r;
-    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
-    return r;
-}
-__device__ __forceinline__ uint32_t hsub2(uint32_t a, uint32_t b) {
-    uint32_t r;
-    asm("sub.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-    return r;
-}
-
-// The eight limbs of X (|X| <= 2^62) as f16 values, limb k in half k:
-// X = sum_{k<7} l_k 2^(8k) + l_7 2^56 with l_0..l_6 in [0, 255] and l_7 in
-// [-64, 64].  The bytes of X + 2^62 are those limbs, the top one plus 64;
-// byte b becomes the f16 1024 + b (exponent bits 0x64 above it) and then the
-// integer b by one exact subtraction per pair.
-__device__ __forceinline__ uint4 to_limbs(long long X) {
-    const unsigned long long Y = (unsigned long long)X + (1ull << 62);
-    const uint32_t lo = uint32_t(Y), hi = uint32_t(Y >> 32);
-    return make_uint4(hsub2(prmt(lo, 0x64646464u, 0x4140u), 0x64006400u),
-                      hsub2(prmt(lo, 0x64646464u, 0x4342u), 0x64006400u),
-                      hsub2(prmt(hi, 0x64646464u, 0x4140u), 0x64006400u),
-                      hsub2(prmt(hi, 0x64646464u, 0x4342u), 0x64406400u));
-}
-
-struct Arena {
-    const int32_t* perm;   // clustered position -> source index
-    const int32_t* iperm;  // source index -> clustered position
-    const LowRankDesc* lr;
-    const DenseDesc* dd;
-    const uint8_t* comp_w;
-    const double* comp_s;
-    const ColTask* tasks;
-    const TaskRec* task_rec;
-    const uint8_t* qcodes;
-    const uint8_t* pcodes;
-    const double* dense;
-    const RowTile* tiles;
-    const TileDense* tdense;
-    const RowUnit* units;
-    const uint8_t* kp_info;
-    const SlotRec* slot_rec;
-    const TaskDest* task_dest;
-    const uint32_t* row_steps;
-    const double* comp_sl;  // s^P per component
-    const double* comp_sr;  // s^Q per component
-};
-
-struct Work {
-    double* xc;        // [rhs][n]            x in clustered order (FP64)
-    int* xblk;         // [rhs][nblk]         largest exponent field of x per prep block
-    int* xe;           // [rhs]               largest exponent field of x
-    uint4* xq;         // [rhs][n_pad]        limbs of X (zero past n)
-    long long* lsplit; // [rhs][n_split*33][8] per-limb sums sum_i c_ij limb_l(X_i) of split tasks'
-                       //                     components (rows split_id*33 + j; zeroed by prep)
-    int* split_cnt;    // [rhs][n_split]      finished parts of each split task (zeroed by prep)
-    uint4* blimb;      // [rhs][n_slots]      row-side B rows: limbs of U
-    uint4* plr;        // [rhs][n_tiles][kTileUnits][16] low-rank row sums of each row unit (128-bit)
-    double* pdense;    // [rhs][n_dslices][64] dense diagonal row sums per dense slice
-};
-
-// -------------------------------------------------- bulk copies (TMA)
-
-__device__ __forceinline__ unsigned smem_u32(const void* p) { return unsigned(__cvta_generic_to_shared(p)); }
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_init_fence() {
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-}
-// Arrive once and expect `bytes` more bytes of transactions on this phase.
-__device__ __forceinline__ void mbar_arrive_expect(uint64_t* bar, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-}
-// Potentially blocking test of a phase: the thread waits until the phase
-// completes or a system-dependent time limit passes (measured faster than an
-// explicit suspend-time hint, which delays the wake-up).
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, unsigned parity) {
-    unsigned ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// Bounded wait: gives up (returns false) after `limit` tests (kWaitLimit:
-// seconds at most) instead of hanging; callers record the failure in the
-// status word, stop issuing copies, give the copies already issued one more
-// bounded wait each and return (best effort: a copy still outstanding after
-// that wait is abandoned with the block).
-constexpr int kWaitLimit = 1 << 22;
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity, int limit = kWaitLimit) {
-    for (int i = 0; i < limit; ++i)
-        if (mbar_try_wait(bar, parity)) return true;
-    return false;
-}
-// Order this thread's (and, after a warp barrier, its warp's) earlier generic
-// accesses to shared memory before later asynchronous-proxy writes to it.
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
-// One-dimensional bulk copy global -> shared (16-byte aligned, bytes % 16 == 0),
-// completing on `bar`.
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
-            smem_u32(dst)),
-        "l"(src), "r"(bytes), "r"(smem_u32(bar))
-        : "memory");
-}
-
-// Programmatic dependent launch: a kernel lets its successor start early
-// (launch_dependents) and waits for its predecessor's results (wait) only
-// where it first reads them; without the launch attribute both are no-ops.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Pipeline depth and CTAs per SM of the two streaming kernels (measured:
 // two stages per warp and two CTAs of 8 warps per SM; capping registers for a
@@ -223,14 +80,6 @@ constexpr int kColPipeSmem = kWarps * kColStages * kColSlotBytes;
 constexpr int kStagedUnits = 24;
 constexpr int kRowPipeSmem = kWarps * kRowStages * kRowSlotBytes;
 
-// Status bits written by the kernels (status word of the apply).
-constexpr int kStatusNonfinite = QH_STATUS_NONFINITE;
-constexpr int kStatusTimeout = QH_STATUS_TIMEOUT;
-
-__device__ __forceinline__ void flag_timeout(int* status) {
-    if (status) atomicOr(status, kStatusTimeout);
-}
-
 // Test aid for the bounded wait: one warp waits, `polls` tests at most, on an
 // mbarrier that nothing ever completes (no copy is issued, so giving up
 // leaves nothing in flight) and records the timeout in the status word
@@ -246,209 +95,7 @@ __global__ void wait_timeout_kernel(int polls, int* status) {
     if (!ok && threadIdx.x == 0) flag_timeout(status);
 }
 
-// round(v * 2^k) for a 128-bit integer v, as a double, with integer
-// operations only (round to nearest even; results outside the normal range
-// take the slow path).
-__device__ __forceinline__ double i128_ldexp(__int128 v, int k) {
-    if (v == 0) return 0.0;
-    const bool neg = v < 0;
-    const unsigned __int128 a = neg ? (unsigned __int128)(-v) : (unsigned __int128)v;
-    const unsigned long long hi = (unsigned long long)(a >> 64), lo = (unsigned long long)a;
-    const int nbits = hi ? 128 - __clzll(hi) : 64 - __clzll(lo);
-    unsigned long long mant;
-    int e;
-    if (nbits <= 53) {
-        mant = lo << (53 - nbits);
-        e = nbits - 53;
-    } else {
-        const int sh = nbits - 53;
-        const unsigned __int128 q = a >> sh;
-        const unsigned __int128 rem = a - (q << sh);
-        const unsigned __int128 half = (unsigned __int128)1 << (sh - 1);
-        mant = (unsigned long long)q;
-        if (rem > half || (rem == half && (mant & 1))) ++mant;
-        e = sh;
-        if (mant >> 53) {
-            mant >>= 1;
-            ++e;
-        }
-    }
-    const int E = e + k + 52 + 1023;
-    if (E <= 0 || E >= 2047) return scalbn(neg ? -double(mant) : double(mant), e + k);
-    const unsigned long long bits =
-        ((unsigned long long)neg << 63) | ((unsigned long long)E << 52) | (mant & 0xFFFFFFFFFFFFFULL);
-    return __longlong_as_double((long long)bits);
-}
-
-__device__ __forceinline__ __int128 shfl_xor_i128(__int128 v, int m) {
-    const long long lo = __shfl_xor_sync(0xFFFFFFFFu, (long long)v, m);
-    const long long hi = __shfl_xor_sync(0xFFFFFFFFu, (long long)(v >> 64), m);
-    return ((__int128)hi << 64) | (unsigned long long)lo;
-}
-
-// ------------------------------------------------- tensor-core fragments
-//
-// A digit d enters the MMA as the f16 bit pattern d, i.e. the subnormal
-// d * 2^-24, so a byte or nibble becomes an operand with one permute (bytes)
-// or one shift-and-mask (nibbles); products with the normal-f16 limbs are
-// exact and every accumulator value is an integer times 2^-24 below 1, exact
-// in FP32.
-
-// Byte group word (digits of entries 2t, 2t+1, 2t+8, 2t+9): the f16 pairs of
-// entries (2t, 2t+1) and (2t+8, 2t+9).
-__device__ __forceinline__ uint32_t dig_lo(uint32_t w) { return prmt(w, 0u, 0x4140u); }
-__device__ __forceinline__ uint32_t dig_hi(uint32_t w) { return prmt(w, 0u, 0x4342u); }
-// Nibble group word: pair k = (nibble k, nibble k + 4); k = 0, 1 are k-block
-// 0's pairs (2t, 2t+1) and (2t+8, 2t+9), k = 2, 3 k-block 1's.
-__device__ __forceinline__ uint32_t nib_pair(uint32_t v, int k) { return (v >> (4 * k)) & 0x000F000Fu; }
-
-// d += A * B for one 16x8x16 step (A: rows g, g+8 x k 2t.., 2t+8..).
-__device__ __forceinline__ void mma_dig(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                        uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3},{%4,%5,%6,%7},{%8,%9},{%0,%1,%2,%3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-// B fragments of two k-blocks from 32 rows of 16 bytes (limbs of 32 entries
-// or components) at a 16-byte-aligned shared address: lane l points at row l.
-__device__ __forceinline__ void limb_frags(uint32_t row_addr, uint32_t (&b)[4]) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3])
-                 : "r"(row_addr)
-                 : "memory");
-}
-
-// One group (rows g and g+8 of a 16-row fragment pair of k-blocks, in
-// shared memory at grp) into d.  Byte rows are 32 bytes, nibble rows 16; rows
-// >= `rows` are zero.  Plain loads (ordered after the stage's mbarrier wait,
-// which clobbers memory) and non-volatile MMAs leave the compiler free to
-// overlap one group's loads with the previous group's MMAs.
-__device__ __forceinline__ void group_mma(float (&d)[4], const uint8_t* grp, bool nib, int rows, int g, int t,
-                                          const uint32_t (&b)[4]) {
-    if (nib) {
-        const uint32_t v0 = g < rows ? *reinterpret_cast<const uint32_t*>(grp + g * 16 + 4 * t) : 0u;
-        const uint32_t v1 = g + 8 < rows ? *reinterpret_cast<const uint32_t*>(grp + (g + 8) * 16 + 4 * t) : 0u;
-        mma_dig(d, nib_pair(v0, 0), nib_pair(v1, 0), nib_pair(v0, 1), nib_pair(v1, 1), b[0], b[1]);
-        mma_dig(d, nib_pair(v0, 2), nib_pair(v1, 2), nib_pair(v0, 3), nib_pair(v1, 3), b[2], b[3]);
-    } else {
-        const uint2 w0 = g < rows ? *reinterpret_cast<const uint2*>(grp + g * 32 + 8 * t) : make_uint2(0u, 0u);
-        const uint2 w1 =
-            g + 8 < rows ? *reinterpret_cast<const uint2*>(grp + (g + 8) * 32 + 8 * t) : make_uint2(0u, 0u);
-        mma_dig(d, dig_lo(w0.x), dig_lo(w1.x), dig_hi(w0.x), dig_hi(w1.x), b[0], b[1]);
-        mma_dig(d, dig_lo(w0.y), dig_lo(w1.y), dig_hi(w0.y), dig_hi(w1.y), b[2], b[3]);
-    }
-}
-
-// The top plane of a column task: stored digits s = d + 2^(t-1) become the
-// signed digit d as a normal f16 (1024 + s, minus hb = 1024 + 2^(t-1) in both
-// halves), so no offset correction is needed on the column side.
-__device__ __forceinline__ uint32_t top_lo(uint32_t w, uint32_t hb) { return hsub2(prmt(w, 0x64646464u, 0x4140u), hb); }
-__device__ __forceinline__ uint32_t top_hi(uint32_t w, uint32_t hb) { return hsub2(prmt(w, 0x64646464u, 0x4342u), hb); }
-__device__ __forceinline__ uint32_t top_nib(uint32_t v, int k, uint32_t hb) {
-    return hsub2(nib_pair(v, k) | 0x64006400u, hb);
-}
-__device__ __forceinline__ void group_mma_top(float (&d)[4], const uint8_t* grp, bool nib, int rows, int g, int t,
-                                              const uint32_t (&b)[4], uint32_t hb) {
-    // rows past `rows` contribute zero: their operands are forced to +0.0
-    const bool in0 = g < rows, in1 = g + 8 < rows;
-    if (nib) {
-        const uint32_t v0 = in0 ? *reinterpret_cast<const uint32_t*>(grp + g * 16 + 4 * t) : 0u;
-        const uint32_t v1 = in1 ? *reinterpret_cast<const uint32_t*>(grp + (g + 8) * 16 + 4 * t) : 0u;
-        uint32_t a[8];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            a[k] = in0 ? top_nib(v0, k, hb) : 0u;
-            a[4 + k] = in1 ? top_nib(v1, k, hb) : 0u;
-        }
-        mma_dig(d, a[0], a[4], a[1], a[5], b[0], b[1]);
-        mma_dig(d, a[2], a[6], a[3], a[7], b[2], b[3]);
-    } else {
-        const uint2 w0 = in0 ? *reinterpret_cast<const uint2*>(grp + g * 32 + 8 * t) : make_uint2(0u, 0u);
-        const uint2 w1 = in1 ? *reinterpret_cast<const uint2*>(grp + (g + 8) * 32 + 8 * t) : make_uint2(0u, 0u);
-        const uint32_t a0 = in0 ? top_lo(w0.x, hb) : 0u, a2 = in0 ? top_hi(w0.x, hb) : 0u;
-        const uint32_t a4 = in0 ? top_lo(w0.y, hb) : 0u, a6 = in0 ? top_hi(w0.y, hb) : 0u;
-        const uint32_t a1 = in1 ? top_lo(w1.x, hb) : 0u, a3 = in1 ? top_hi(w1.x, hb) : 0u;
-        const uint32_t a5 = in1 ? top_lo(w1.y, hb) : 0u, a7 = in1 ? top_hi(w1.y, hb) : 0u;
-        mma_dig(d, a0, a1, a2, a3, b[0], b[1]);
-        mma_dig(d, a4, a5, a6, a7, b[2], b[3]);
-    }
-}
-
-// The top plane of a row k-pair: stored digits s = d + 2^(t-1) become the
-// signed digit d on the lower planes' scale, d 2^-24 (a subnormal f16 for
-// |d| < 1024): the f16 with exponent field 1 and mantissa s is (1024 + s)
-// 2^-24, minus hb = (1024 + 2^(t-1)) 2^-24 in both halves, exactly.
-__device__ __forceinline__ uint32_t rtop_lo(uint32_t w, uint32_t hb) { return hsub2(prmt(w, 0x04040404u, 0x4140u), hb); }
-__device__ __forceinline__ uint32_t rtop_hi(uint32_t w, uint32_t hb) { return hsub2(prmt(w, 0x04040404u, 0x4342u), hb); }
-__device__ __forceinline__ uint32_t rtop_nib(uint32_t v, int k, uint32_t hb) {
-    return hsub2(nib_pair(v, k) | 0x04000400u, hb);
-}
-__device__ __forceinline__ void group_mma_rtop(float (&d)[4], const uint8_t* grp, bool nib, int g, int t,
-                                               const uint32_t (&b)[4], uint32_t hb) {
-    if (nib) {
-        const uint32_t v0 = *reinterpret_cast<const uint32_t*>(grp + g * 16 + 4 * t);
-        const uint32_t v1 = *reinterpret_cast<const uint32_t*>(grp + (g + 8) * 16 + 4 * t);
-        mma_dig(d, rtop_nib(v0, 0, hb), rtop_nib(v1, 0, hb), rtop_nib(v0, 1, hb), rtop_nib(v1, 1, hb), b[0], b[1]);
-        mma_dig(d, rtop_nib(v0, 2, hb), rtop_nib(v1, 2, hb), rtop_nib(v0, 3, hb), rtop_nib(v1, 3, hb), b[2], b[3]);
-    } else {
-        const uint2 w0 = *reinterpret_cast<const uint2*>(grp + g * 32 + 8 * t);
-        const uint2 w1 = *reinterpret_cast<const uint2*>(grp + (g + 8) * 32 + 8 * t);
-        mma_dig(d, rtop_lo(w0.x, hb), rtop_lo(w1.x, hb), rtop_hi(w0.x, hb), rtop_hi(w1.x, hb), b[0], b[1]);
-        mma_dig(d, rtop_lo(w0.y, hb), rtop_lo(w1.y, hb), rtop_hi(w0.y, hb), rtop_hi(w1.y, hb), b[2], b[3]);
-    }
-}
-
-// Digits of rows g, g+8 of a group as integers, in the order the MMA sees
-// them (for validation): out[half][kb*4 + s], s = entries 2t, 2t+1, 2t+8, 2t+9.
-__device__ __forceinline__ void group_digits(const uint8_t* grp, bool nib, int rows, int g, int t,
-                                             uint32_t (&out)[2][8]) {
-    uint32_t r[2][4];  // [half][kb0 lo, kb0 hi, kb1 lo, kb1 hi]
-    if (nib) {
-        const uint32_t v0 = g < rows ? *reinterpret_cast<const uint32_t*>(grp + g * 16 + 4 * t) : 0u;
-        const uint32_t v1 = g + 8 < rows ? *reinterpret_cast<const uint32_t*>(grp + (g + 8) * 16 + 4 * t) : 0u;
-        for (int k = 0; k < 4; ++k) {
-            r[0][k] = nib_pair(v0, k);
-            r[1][k] = nib_pair(v1, k);
-        }
-    } else {
-        const uint2 w0 = g < rows ? *reinterpret_cast<const uint2*>(grp + g * 32 + 8 * t) : make_uint2(0u, 0u);
-        const uint2 w1 =
-            g + 8 < rows ? *reinterpret_cast<const uint2*>(grp + (g + 8) * 32 + 8 * t) : make_uint2(0u, 0u);
-        r[0][0] = dig_lo(w0.x), r[0][1] = dig_hi(w0.x), r[0][2] = dig_lo(w0.y), r[0][3] = dig_hi(w0.y);
-        r[1][0] = dig_lo(w1.x), r[1][1] = dig_hi(w1.x), r[1][2] = dig_lo(w1.y), r[1][3] = dig_hi(w1.y);
-    }
-    for (int hh = 0; hh < 2; ++hh)
-        for (int k = 0; k < 4; ++k) {
-            // pair k: k-block k >> 1, slots (2(k&1), 2(k&1) + 1)
-            out[hh][(k >> 1) * 4 + 2 * (k & 1)] = r[hh][k] & 0xFFFFu;
-            out[hh][(k >> 1) * 4 + 2 * (k & 1) + 1] = r[hh][k] >> 16;
-        }
-}
-// Entry (within a 32-entry k-pair) of slot s of k-block kb for thread t.
-__device__ __forceinline__ int slot_entry(int kb, int s, int t) { return 16 * kb + 2 * t + (s & 1) + 8 * (s >> 1); }
-
-// Exact integers sum(D * 2^24) of a plane's accumulators, folded into 64-bit
-// sums at weight 2^(8m).
-__device__ __forceinline__ long long fold(float d, int m) {
-    return (long long)__float2int_rn(d * 16777216.0f) << (8 * m);
-}
-
-// Widths a code may have (the reference's writer allows 2..32).
-#define QH_WIDTH_CASES(X) \
-    X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16) X(17) \
-    X(18) X(19) X(20) X(21) X(22) X(23) X(24) X(25) X(26) X(27) X(28) X(29) X(30) X(31) X(32)
-
 // ---------------------------------------------------------------- kernels
-
-__device__ __forceinline__ void st_i128(uint4* p, __int128 v) {
-    *p = make_uint4(uint32_t(v), uint32_t(v >> 32), uint32_t(v >> 64), uint32_t(v >> 96));
-}
-__device__ __forceinline__ __int128 ld_i128(const uint4* p) {
-    const uint4 v = __ldcg(p);
-    return (__int128)(((unsigned __int128)v.w << 96) | ((unsigned __int128)v.z << 64) |
-                      ((unsigned __int128)v.y << 32) | v.x);
-}
 
 // Block (bx, p) of 8 warps: source entries 256bx .. 256bx+255 of rhs column
 // p, read in order (coalesced; x may be the caller's host memory, read over
@@ -659,8 +306,11 @@ __device__ __forceinline__ void dense_unit(const Arena& A, const Work& W, const 
 // signed); the FP32 sums are folded into 64-bit integers every 8 chunks
 // (before any can reach 2^24).  At the unit's end the limbs and planes are
 // combined into exact 128-bit sums t_j = sum_i c_ij X_i (lane j: component j,
-// through shared memory), u_j = (s^P s^Q) t_j 2^(xe - 1022 - kFixBits), and
-// the B rows of u_j on each consuming tile's exponent are written.  Dense
+// through shared memory), u_j in fixed point (comp_fixed: integer shifts and
+// one 64 x 64-bit product instead of a 128-bit to FP64 conversion, an FP64
+// product and a conversion back per destination -- 85.2 -> 82.9 us per apply
+// at n = 32768), and the B rows of u_j on each consuming tile's exponent are
+// written.  Dense
 // units (width 0) are computed in FP64 by dense_unit.
 __global__ void __launch_bounds__(kWarps * 32, QH_COL_CTAS) column_kernel(Arena A, Work W, const int* __restrict__ warp_off,
                                                                 int n_pad, int rhs, int n_split, int n_slots,
@@ -765,14 +415,18 @@ __global__ void __launch_bounds__(kWarps * 32, QH_COL_CTAS) column_kernel(Arena 
         defer = false;
         if (lane == 0)
             for (int i = 0; i < npend; ++i) bulk_load(pend_dst[i], pend_src[i], pend_bytes[i], bar + pend_slot[i]);
-        const int xe0 = W.xe[0];
-        // this lane's component scale and first B row record, loaded when a
+        // this lane's component record and first B row record, loaded when a
         // unit starts (the record by an asynchronous copy into shared
         // memory) and used at its end
-        double rec = 0.0;
+        int shift = 1;
+        unsigned long long kappa = 0;
         int2* my_td = &s_td[warp][lane];
         auto load_rec = [&]() {
-            if (lane < dc.count) rec = __ldg(&A.task_rec[dc.comp_idx + lane].scale);
+            if (lane < dc.count) {
+                const uint4 r = __ldg(reinterpret_cast<const uint4*>(A.task_rec + dc.comp_idx + lane));
+                shift = int((r.y >> 8) & 255u);
+                kappa = ((unsigned long long)r.w << 32) | r.z;
+            }
             if (lane < dc.ndest) cp_async8(my_td, A.task_dest + dc.dest0 + lane);
         };
         load_rec();
@@ -820,7 +474,6 @@ __global__ void __launch_bounds__(kWarps * 32, QH_COL_CTAS) column_kernel(Arena 
                 // refilled before the next issue) and let lane j finish row j;
                 // a part of a split task adds its sums exactly with atomics and
                 // the part that finishes last finishes the rows.
-                const int xe = cp == 0 ? xe0 : W.xe[cp];
                 long long* st = reinterpret_cast<long long*>(const_cast<uint8_t*>(slot));
                 bool finish = true;
                 if (dc.nparts == 1) {
@@ -864,17 +517,17 @@ __global__ void __launch_bounds__(kWarps * 32, QH_COL_CTAS) column_kernel(Arena 
                     for (int l = 32 + 16 * lane; l < dc.ndest; l += 512)  // the rest of a long B row list
                         prefetch_l2(A.task_dest + dc.dest0 + l);
                     __syncwarp();
-                    // lane j: u of component row j
-                    double u = 0.0;
+                    // lane j: u of component row j in fixed point
+                    long long v = 0;
                     if (lane < dc.count) {
                         const longlong2* r2 = reinterpret_cast<const longlong2*>(st + lane * 8);
                         __int128 S = 0;
 #pragma unroll
                         for (int l = 0; l < 4; ++l) {
-                            const longlong2 v = r2[l];
-                            S += ((__int128)v.x << (16 * l)) + ((__int128)v.y << (16 * l + 8));
+                            const longlong2 w = r2[l];
+                            S += ((__int128)w.x << (16 * l)) + ((__int128)w.y << (16 * l + 8));
                         }
-                        u = xe ? i128_ldexp(S, xe - 1022 - kFixBits) * rec : 0.0;
+                        v = comp_fixed(S, shift, kappa);
                     }
                     // the task's B rows, lanes over the (component, slot)
                     // pairs: U on the tile's exponent and its limbs
@@ -890,12 +543,9 @@ __global__ void __launch_bounds__(kWarps * 32, QH_COL_CTAS) column_kernel(Arena 
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
                             if (d0 + 32 * j >= dc.ndest) break;
-                            const double ud = __shfl_sync(0xFFFFFFFFu, u, (td[j].y >> 16) & 31);
-                            if (td[j].x >= 0) {
-                                const int ce = int(int16_t(td[j].y & 0xFFFF));
-                                const long long U = to_fixed(ud, xe + ce);  // (0 for 0)
-                                W.blimb[(long long)cp * n_slots + td[j].x] = to_limbs(U);
-                            }
+                            const long long vd = __shfl_sync(0xFFFFFFFFu, v, (td[j].y >> 16) & 31);
+                            if (td[j].x >= 0)
+                                W.blimb[(long long)cp * n_slots + td[j].x] = to_limbs(tile_fixed(vd, td[j].y & 63));
                         }
                     }
                 }
