@@ -508,6 +508,9 @@ Layout build_layout(const HostMatrix& m) {
     std::vector<SlotRec> slot_rec;   // each B row slot's component, shift and width
     std::vector<std::vector<std::pair<int32_t, int32_t>>> comp_dest(m.width.size());  // per component: (slot, tile)
     std::vector<uint32_t> row_steps; // pipeline steps of the row units
+    std::vector<std::pair<int64_t, TcRowItem>> row_items;  // (steps, item)
+    std::vector<TcStep> tc_steps;
+    int32_t n_parts = 0;
     struct RowComp {
         int w;
         int32_t comp;
@@ -556,6 +559,7 @@ Layout build_layout(const HostMatrix& m) {
                 ktop[size_t(kp)] = tb;
                 kp_info.push_back(uint8_t(planes | (top_is_nibble(w) ? 8 : 0) | ((tb - 1) << 4)));
             }
+            auto hkps = [&](int32_t h) { return (Kp - h + T.hsplit - 1) / T.hsplit; };  // k-pairs of split h
             // B row slots: k split h's k-pairs contiguously
             std::vector<int64_t> hslot(size_t(T.hsplit), 0);
             for (int32_t h = 0; h < T.nh; ++h) {
@@ -574,6 +578,7 @@ Layout build_layout(const HostMatrix& m) {
                 }
                 n_slots += 32 * int64_t((Kp - h + T.hsplit - 1) / T.hsplit);
             }
+            int64_t tile_code[4][kTileUnits] = {};
             // streams (q, h): groups of 16 rows
             for (int32_t q = 0; q < T.qrows; ++q)
                 for (int32_t h = 0; h < T.nh; ++h) {
@@ -644,8 +649,40 @@ Layout build_layout(const HostMatrix& m) {
                             }
                             bytes += int64_t(16 * rb);
                         }
+                    tile_code[size_t(q)][size_t(h)] = U.code_off;
                     units.push_back({bytes + int64_t(U.nkps) * 512, U});
                 }
+            // the tensor-memory kernel's view of the tile
+            T.part0 = n_parts;
+            T.parts = (rows <= 32 ? 32 : 64) << 16;
+            if (T.nh > 0) {
+                const int32_t steps_h = (hkps(0) + 1) / 2;
+                const int32_t per = std::max<int32_t>(1, (kRowItemSteps + steps_h - 1) / steps_h);  // splits per item
+                for (int32_t h0 = 0; h0 < T.nh; h0 += per) {
+                    TcRowItem I{int32_t(tc_steps.size()), 0, (rows <= 32 ? 32 : 64) | T.qrows << 8, n_parts++};
+                    ++T.parts;
+                    for (int32_t h = h0; h < std::min(T.nh, h0 + per); ++h) {
+                        int64_t off = 0;
+                        for (int32_t i = 0; i < hkps(h); i += 2) {
+                            TcStep S{};
+                            for (int q = 0; q < T.qrows; ++q)
+                                S.code[q] = uint32_t((tile_code[q][h] + off) / 256);
+                            S.slot = int32_t(hslot[size_t(h)]) + 32 * i;
+                            S.nslots = 32 * std::min(2, hkps(h) - i);
+                            for (int j = 0; j < 2 && i + j < hkps(h); ++j) {
+                                const size_t kp = size_t(h + (i + j) * T.hsplit);
+                                S.info |= uint32_t(kp_info[size_t(kp_off) + kp]) << (8 * j);
+                                off += 512 * kplanes[kp] - (knib[kp] ? 256 : 0);
+                            }
+                            if (i % 4 == 2 || i + 2 >= hkps(h)) S.info |= kSegmentEnd;
+                            tc_steps.push_back(S);
+                        }
+                    }
+                    tc_steps.back().info |= kItemEnd;
+                    I.nsteps = int32_t(tc_steps.size()) - I.step0;
+                    row_items.push_back({I.nsteps, I});
+                }
+            }
             if (T.qrows * T.nh + T.ndense == 0) throw runtime_error("row tile without blocks");
             tiles.push_back(T);
         }
@@ -720,7 +757,61 @@ Layout build_layout(const HostMatrix& m) {
     L.n_slots = int32_t(n_slots);
     L.n_tdense = int32_t(tdense.size());
     L.stored_p_bytes = pcodes.size();
-    if (qcodes.size() >= (1ull << 42) || pcodes.size() >= (1ull << 42))
+    // ---- work lists of the tensor-memory kernels.  Column side: the tasks of
+    // a range by planes and size, four to an item; costliest items first.
+    std::vector<TcItem> tc_items;
+    std::vector<TcTask> tc_tasks;
+    std::vector<DenseUnit> dense_units;
+    {
+        std::vector<int32_t> idx;
+        for (size_t t = 0; t < tasks.size(); ++t) {
+            const ColTask& T = tasks[t];
+            if (T.width) idx.push_back(int32_t(t));
+            else dense_units.push_back({T.col0, T.stride, T.comp_idx, T.chunk0, T.n, {0, 0, 0}});
+        }
+        auto key = [&](int32_t t) {
+            const ColTask& T = tasks[size_t(t)];
+            return std::make_pair(std::make_pair(T.col0, T.n), std::make_pair(T.chunk0, -code_planes(T.width)));
+        };
+        std::stable_sort(idx.begin(), idx.end(), [&](int32_t a, int32_t b) {
+            const auto ka = key(a), kb = key(b);
+            return ka != kb ? ka < kb : tasks[size_t(a)].count > tasks[size_t(b)].count;
+        });
+        std::vector<std::pair<int64_t, std::pair<size_t, size_t>>> groups;  // (cost, tasks [a, b) of idx)
+        for (size_t i = 0; i < idx.size();) {
+            size_t j = i;
+            while (j < idx.size() && j - i < 4 && key(idx[i]) == key(idx[j])) ++j;
+            const ColTask& T = tasks[size_t(idx[i])];
+            // a fixed part per item, then planes x 64-entry blocks
+            groups.push_back({4 + int64_t((T.nchunks + 1) / 2) * code_planes(T.width), {i, j}});
+            i = j;
+        }
+        std::stable_sort(groups.begin(), groups.end(),
+                         [](const auto& a, const auto& b) { return a.first > b.first; });
+        for (const auto& g : groups) {
+            const ColTask& T0 = tasks[size_t(idx[g.second.first])];
+            tc_items.push_back({T0.col0, T0.chunk0, T0.nchunks,
+                                code_planes(T0.width) | int32_t(g.second.second - g.second.first) << 8});
+            for (size_t k = 0; k < 4; ++k) {
+                if (g.second.first + k >= g.second.second) {
+                    tc_tasks.push_back(TcTask{0, 0, 0, 0, -1, 1, 0});
+                    continue;
+                }
+                const ColTask& T = tasks[size_t(idx[g.second.first + k])];
+                tc_tasks.push_back({T.off + int64_t(T.chunk0) * T.stride, T.stride, T.comp_idx, T.count | T.width << 8,
+                                    T.split_id, T.nparts, 0});
+            }
+        }
+    }
+    std::stable_sort(row_items.begin(), row_items.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
+    std::vector<TcRowItem> tc_row_items;
+    for (const auto& r : row_items) tc_row_items.push_back(r.second);
+    L.n_tc_items = int32_t(tc_items.size());
+    L.n_tc_row_items = int32_t(tc_row_items.size());
+    L.n_dense_units = int32_t(dense_units.size());
+    L.n_parts = n_parts;
+    // (row code offsets are kept in 256-byte units)
+    if (qcodes.size() >= (1ull << 42) || pcodes.size() >= (1ull << 40))
         throw overflow_error("packed factors too large for the device layout");
 
     // ---- arena sections, each 256-byte aligned.
@@ -752,6 +843,11 @@ Layout build_layout(const HostMatrix& m) {
     S.row_steps = place(4 * row_steps.size());
     S.comp_sl = place(8 * C);
     S.comp_sr = place(8 * C);
+    S.tc_items = place(sizeof(TcItem) * tc_items.size());
+    S.tc_tasks = place(sizeof(TcTask) * tc_tasks.size());
+    S.dense_units = place(sizeof(DenseUnit) * dense_units.size());
+    S.tc_row_items = place(sizeof(TcRowItem) * tc_row_items.size());
+    S.tc_steps = place(sizeof(TcStep) * tc_steps.size());
     S.total = off;
 
     L.arena.assign(S.total, 0);
@@ -781,6 +877,14 @@ Layout build_layout(const HostMatrix& m) {
     if (!row_steps.empty()) std::memcpy(A.data() + S.row_steps, row_steps.data(), 4 * row_steps.size());
     if (!dense_cm.empty()) std::memcpy(A.data() + S.dense, dense_cm.data(), 8 * dense_cm.size());
     if (!tiles.empty()) std::memcpy(A.data() + S.tiles, tiles.data(), sizeof(RowTile) * tiles.size());
+    auto put = [&](size_t at, const auto& v) {
+        if (!v.empty()) std::memcpy(A.data() + at, v.data(), sizeof(v[0]) * v.size());
+    };
+    put(S.tc_items, tc_items);
+    put(S.tc_tasks, tc_tasks);
+    put(S.dense_units, dense_units);
+    put(S.tc_row_items, tc_row_items);
+    put(S.tc_steps, tc_steps);
     if (!tdense.empty()) std::memcpy(A.data() + S.tdense, tdense.data(), sizeof(TileDense) * tdense.size());
     return L;
 }

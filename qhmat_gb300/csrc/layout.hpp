@@ -171,7 +171,8 @@ struct DenseDesc {
 struct RowTile {
     int32_t row0, rows, qrows, hsplit;
     int32_t nh, ndense, dense0, c_exp;
-    int32_t ds0, nds, pad[2];
+    int32_t ds0, nds;
+    int32_t part0, parts;  // row items' partial sums; parts | rs << 16
 };
 static_assert(sizeof(RowTile) == 48, "RowTile layout");
 // A dense diagonal block's part in a row tile: value (tile row r, column k)
@@ -202,6 +203,52 @@ struct SlotRec {
     int32_t comp, info;
 };
 
+// ---- work lists of the tensor-memory kernels (tc.cu), over the same codes.
+//
+// Column side: an item is up to four tasks (parts) of <= 32 components that
+// share a column range, a run of chunks and a number of digit planes: task s
+// gives rows 32s .. of a 128-row MMA tile.
+struct TcItem {
+    int32_t col0, chunk0, nchunks, info;  // info: planes | tasks << 8
+};
+static_assert(sizeof(TcItem) == 16, "TcItem layout");
+// A task of an item: `off` is its first chunk's byte in the codes, chunks are
+// `stride` bytes apart; info = components | width << 8; split: the split
+// task's index (parts add their sums) or -1.
+struct TcTask {
+    int64_t off;
+    int32_t stride, comp_idx;
+    int32_t info, split, nparts, pad;
+};
+static_assert(sizeof(TcTask) == 32, "TcTask layout");
+// Columns [k0, k0 + cols) of tdense[tdense] of a row tile, row-sum slice `slice`.
+struct DenseUnit {
+    int32_t tdense, tile, slice, k0, cols, pad[3];
+};
+static_assert(sizeof(DenseUnit) == 32, "DenseUnit layout");
+// Row side: an item is a run of steps, each two k-pairs (64 slots) of one k
+// split of a tile; its row sums are partial `part`.  The MMA tile's 128 rows
+// are `rs` (32 or 64) tile rows for each of 128 / rs digit planes; qrows: the
+// tile's 16-row M-tiles.
+struct TcRowItem {
+    int32_t step0, nsteps, shape, part;  // shape: rs | qrows << 8
+};
+static_assert(sizeof(TcRowItem) == 16, "TcRowItem layout");
+// `code[q]`: the step's digit groups of M-tile q (byte offset / 256); `slot`:
+// its first B row slot, `nslots` of them; info: the k-pairs' info bytes
+// (second << 8, 0: none), kSegmentEnd on the last step of an accumulator
+// segment (at most two steps, one split), kItemEnd on the item's last step.
+struct TcStep {
+    uint32_t code[4];
+    int32_t slot, nslots;
+    uint32_t info, pad;
+};
+static_assert(sizeof(TcStep) == 32, "TcStep layout");
+constexpr uint32_t kSegmentEnd = 1u << 16, kItemEnd = 1u << 17;
+// Steps a row item holds at least where its tile has them (shorter ones would
+// be dominated by their pipeline's ends).
+constexpr int kRowItemSteps = 8;
+
 // Bytes of one column-side shared-memory stage (code groups and x rows of
 // the step's chunks); one row-side stage (code groups and B rows).  Two
 // stages per warp, eight warps per CTA and two CTAs per SM: 6144-byte stages
@@ -223,7 +270,7 @@ inline bool top_is_nibble(int w) { return w - 8 * (code_planes(w) - 1) <= 4; }
 // Byte offsets of each section inside the device arena.
 struct Sections {
     size_t perm, iperm, lr, dd, comp_w, comp_s, tasks, task_rec, task_dest, qcodes, pcodes, dense, tiles, tdense, units,
-        kp_info, slot_rec, row_steps, comp_sl, comp_sr;
+        kp_info, slot_rec, row_steps, comp_sl, comp_sr, tc_items, tc_tasks, dense_units, tc_row_items, tc_steps;
     size_t total;
 };
 
@@ -232,6 +279,8 @@ struct Layout {
     int32_t n_lr = 0, n_dense = 0, n_comp = 0, n_tiles = 0, n_chunks = 0;
     int32_t n_tasks = 0, n_split = 0, max_parts = 1;
     int32_t n_units = 0, n_slots = 0, n_tdense = 0, n_dest = 0, n_dslices = 0;
+    int32_t n_tc_items = 0, n_tc_row_items = 0, n_dense_units = 0;
+    int32_t n_parts = 0;   // row-side partial sums (128 rows each)
     std::vector<uint8_t> arena;  // host image of the device arena
     Sections sec{};
     double bound = 0;

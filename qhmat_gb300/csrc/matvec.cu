@@ -29,6 +29,9 @@
 //   combine_kernel     thread per row: dense row sums in column order plus
 //                      the partials -> y (one conversion).
 //
+// Applies of three columns and more take the column, row and combine kernels of
+// tc.cu instead (the same integers on the 5th-generation tensor cores).
+//
 // The only rounding steps are the fixed-point conversions of x and u (2^-63
 // of the column's largest |x|, ~2^-62 of the component's and of the tile's
 // bound on |u|), the product s^P s^Q, and the final FP64 conversions: the
@@ -56,7 +59,7 @@
 #include "batch.hpp"
 #include "errors.hpp"
 #include "layout.hpp"
-#include "plain.hpp"
+#include "tc.hpp"
 
 namespace qhg {
 namespace {
@@ -571,11 +574,6 @@ __global__ void __launch_bounds__(kWarps * 32, QH_COL_CTAS) column_kernel(Arena 
         ++computed;
     }
 }
-
-// A row k-pair's info byte: planes | nibble top plane << 3 | (top bits - 1) << 4.
-// Bytes of its digit groups, and the top plane's conversion constant.
-__device__ __forceinline__ int kp_bytes(int info) { return (info & 7) * 512 - ((info >> 3) & 1) * 256; }
-__device__ __forceinline__ uint32_t kp_hb(int info) { return (0x0400u | (1u << (info >> 4))) * 0x00010001u; }
 
 // A row unit's descriptor (four 16-byte loads, cached in L1).
 struct RowDesc {
@@ -1210,6 +1208,7 @@ int upload(Layout&& L, int device, qh_matrix** out) {
     e = cudaFuncSetAttribute(row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowPipeSmem);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(column_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kColPipeSmem);
+    if (e == cudaSuccess) e = tc_setup();
     if (e != cudaSuccess) {
         delete m;
         return cuda_fail(e, "cudaFuncSetAttribute");
@@ -1238,6 +1237,11 @@ int upload(Layout&& L, int device, qh_matrix** out) {
     m->A.row_steps = reinterpret_cast<const uint32_t*>(base + S.row_steps);
     m->A.comp_sl = reinterpret_cast<const double*>(base + S.comp_sl);
     m->A.comp_sr = reinterpret_cast<const double*>(base + S.comp_sr);
+    m->A.tc_items = reinterpret_cast<const TcItem*>(base + S.tc_items);
+    m->A.tc_tasks = reinterpret_cast<const TcTask*>(base + S.tc_tasks);
+    m->A.dense_units = reinterpret_cast<const DenseUnit*>(base + S.dense_units);
+    m->A.tc_row_items = reinterpret_cast<const TcRowItem*>(base + S.tc_row_items);
+    m->A.tc_steps = reinterpret_cast<const TcStep*>(base + S.tc_steps);
     *out = m;
     return QH_OK;
 }
@@ -1265,15 +1269,15 @@ constexpr size_t kMaxRhsChunk = 65535;
 size_t rhs_chunk(size_t rhs) { return std::min(rhs, kMaxRhsChunk); }
 
 struct WsPlan {
-    size_t xc, xblk, xe, xq, lsplit, cnt, blimb, plr, pdense, total, zero0, zero_bytes;
-    int nblk;
+    size_t xc, xblk, xe, xq, lsplit, cnt, blimb, part, plr, pdense, total, zero0, zero_bytes;
+    int nblk, pv;  // pv > 0: columns of a row of V (the tensor-memory kernels)
 };
 
 // x limbs are read by whole 32-entry chunks: pad past the last chunk.
 size_t padded_order(const Layout& L) { return (L.order + kColChunk - 1) / kColChunk * kColChunk + kColChunk; }
 
-WsPlan ws_plan(const Layout& L, size_t rhs) {
-    WsPlan w;
+WsPlan ws_plan(const Layout& L, size_t rhs, bool tc) {
+    WsPlan w = {};
     size_t off = 0;
     auto take = [&](size_t bytes) {
         const size_t o = off;
@@ -1290,32 +1294,41 @@ WsPlan ws_plan(const Layout& L, size_t rhs) {
     w.xblk = take(4 * size_t(w.nblk) * rhs);
     w.xc = take(8 * L.order * rhs);
     w.xq = take(16 * padded_order(L) * rhs);
-    w.blimb = take(16 * size_t(L.n_slots) * rhs);
-    w.plr = take(16 * 16 * kTileUnits * size_t(L.n_tiles) * rhs);
+    if (tc) {  // V and the row items' sums
+        const int R = tc_columns(int(rhs));
+        w.pv = (int(rhs) + R - 1) / R * R;
+        w.blimb = take(8 * size_t(L.n_comp) * size_t(w.pv));
+        w.part = take(16 * 128 * size_t(L.n_parts) * rhs);
+    } else {  // B rows and row sums of the column-by-column kernels
+        w.blimb = take(16 * size_t(L.n_slots) * rhs);
+        w.plr = take(16 * 16 * kTileUnits * size_t(L.n_tiles) * rhs);
+    }
     w.pdense = take(8 * 64 * size_t(L.n_dslices) * rhs);
     w.total = off;
     return w;
 }
 
-// Workspace of an apply with rhs columns (one column chunk's worth).
-size_t ws_bytes(const Layout& L, size_t rhs) { return ws_plan(L, rhs_chunk(rhs)).total; }
-
-// Launch with programmatic stream serialization (the kernel may start while
-// its predecessor finishes; it waits in-kernel for the predecessor's results).
-template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k, static_cast<KArgs>(args)...);
+// The kernels of an apply of rhs columns: the tensor-memory ones (tc.cu) from
+// three columns on, the column-by-column ones below.  The latter stream and
+// convert every code once per column, the former once per four or eight
+// columns, in steps with a fixed handshake cost.  Whole applies on the device,
+// us, column by column / tensor memory (2-D, leaf 64 unless noted):
+//                        1 column   2          3          4          16
+//   n =  2048 (1-D, 32)  20 / 25    27 / 27    35 / 27    43 / 28    146 / 39
+//   n =  9001 (leaf 32)  43 / 97    77 / 105   112 / 108  150 / 110  526 / 284
+//   n = 16384            43 / 78    75 / 83    115 / 87   153 / 88   556 / 186
+//   n =  8192 (3-D)      54 / 77    95 / 80    138 / 81   179 / 82   644 / 195
+//   n = 32768            81 / 155   146 / -    212 / 177  277 / 179
+// Their workspace must also fit the column-by-column kernels' (which sizes
+// every workspace; V is smaller than B rows wherever a component is read by
+// more than one row tile).
+constexpr size_t kTcColumns = 3;
+bool use_tc(const Layout& L, size_t rhs) {
+    return rhs >= kTcColumns && ws_plan(L, rhs, true).total <= ws_plan(L, rhs, false).total;
 }
+
+// Workspace of an apply with rhs columns (one column chunk's worth).
+size_t ws_bytes(const Layout& L, size_t rhs) { return ws_plan(L, rhs_chunk(rhs), false).total; }
 
 // One chain of launches for columns [c0, c0 + rhs) of x and y (leading
 // dimension ld).
@@ -1324,7 +1337,8 @@ int launch_chunk(const qh_matrix* m, const double* x, double* y, size_t rhs, lon
     const Layout& L = m->L;
     const int n = int(L.order);
     auto* w = static_cast<uint8_t*>(ws);
-    const WsPlan P = ws_plan(L, rhs);
+    const bool tc = use_tc(L, rhs);
+    const WsPlan P = ws_plan(L, rhs, tc);
     Work W;
     W.xc = reinterpret_cast<double*>(w + P.xc);
     W.xblk = reinterpret_cast<int*>(w + P.xblk);
@@ -1333,6 +1347,8 @@ int launch_chunk(const qh_matrix* m, const double* x, double* y, size_t rhs, lon
     W.lsplit = reinterpret_cast<long long*>(w + P.lsplit);
     W.split_cnt = reinterpret_cast<int*>(w + P.cnt);
     W.blimb = reinterpret_cast<uint4*>(w + P.blimb);
+    W.v = reinterpret_cast<long long*>(w + P.blimb);
+    W.part = reinterpret_cast<uint4*>(w + P.part);
     W.plr = reinterpret_cast<uint4*>(w + P.plr);
     W.pdense = reinterpret_cast<double*>(w + P.pdense);
     auto mark = [&](int i) {
@@ -1363,17 +1379,31 @@ int launch_chunk(const qh_matrix* m, const double* x, double* y, size_t rhs, lon
                        n_pad, P.nblk);
     }
     mark(1);
-    if (e == cudaSuccess && L.n_tasks > 0)
-        e = launch_pdl(column_kernel, dim3(unsigned(m->col_grid)), dim3(kWarps * 32), size_t(kColPipeSmem), s, m->A,
-                       W, static_cast<const int*>(m->sched), n_pad, irhs, L.n_split, L.n_slots, n, L.n_dslices, status);
-    mark(2);
-    if (e == cudaSuccess && L.n_units > 0)
-        e = launch_pdl(row_kernel, dim3(unsigned(m->row_grid)), dim3(kWarps * 32), size_t(kRowPipeSmem), s, m->A, W,
-                       static_cast<const int*>(m->sched + m->col_grid * kWarps + 1), irhs, L.n_slots, L.n_tiles,
-                       status);
-    if (e == cudaSuccess)
-        e = launch_pdl(combine_kernel, dim3(unsigned(L.n_tiles), unsigned(rhs)), dim3(64), 0, s, m->A, W, y,
-                       L.n_tiles, L.n_dslices, ld);
+    if (tc) {
+        const TcArgs t{m->A, W, L.n_tc_items, L.n_tc_row_items, L.n_dense_units, L.n_parts, L.n_tiles, irhs, P.pv, n,
+                       n_pad, L.n_split, L.n_dslices, m->sms, y, ld, status};
+        struct Ctx {
+            void* const* ev;
+            cudaStream_t s;
+        } ctx{ev, s};
+        void (*record)(void*, int) = [](void* c, int i) {
+            auto* x = static_cast<Ctx*>(c);
+            cudaEventRecord(static_cast<cudaEvent_t>(x->ev[i]), x->s);
+        };
+        if (e == cudaSuccess) e = tc_launch(t, s, ev ? record : nullptr, &ctx);
+    } else {
+        if (e == cudaSuccess && L.n_tasks > 0)
+            e = launch_pdl(column_kernel, dim3(unsigned(m->col_grid)), dim3(kWarps * 32), size_t(kColPipeSmem), s, m->A,
+                           W, static_cast<const int*>(m->sched), n_pad, irhs, L.n_split, L.n_slots, n, L.n_dslices, status);
+        mark(2);
+        if (e == cudaSuccess && L.n_units > 0)
+            e = launch_pdl(row_kernel, dim3(unsigned(m->row_grid)), dim3(kWarps * 32), size_t(kRowPipeSmem), s, m->A, W,
+                           static_cast<const int*>(m->sched + m->col_grid * kWarps + 1), irhs, L.n_slots, L.n_tiles,
+                           status);
+        if (e == cudaSuccess)
+            e = launch_pdl(combine_kernel, dim3(unsigned(L.n_tiles), unsigned(rhs)), dim3(64), 0, s, m->A, W, y,
+                           L.n_tiles, L.n_dslices, ld);
+    }
     if (e != cudaSuccess) return cuda_fail(e, "CUDA kernel launch");
     mark(3);
     e = cudaGetLastError();
@@ -1523,7 +1553,7 @@ int qh_matrix_stats(const qh_matrix* m, qh_stats* out) {
     out->device_bytes = L.sec.total;
     out->row_tiles = uint64_t(L.n_tiles);
     out->flops_per_rhs = L.flops;
-    const WsPlan P1 = ws_plan(L, 1);
+    const WsPlan P1 = ws_plan(L, 1, false);
     out->launches_per_apply = (P1.nblk <= m->prep_coop_max ? 2 : 3) + (L.n_tasks > 0) + (L.n_units > 0);
     out->host_direct = m->host_direct ? 1 : 0;
     out->left_code_bytes = L.left_code_bytes;

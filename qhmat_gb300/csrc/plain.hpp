@@ -12,6 +12,50 @@
 #include "layout.hpp"
 
 namespace qhg {
+
+struct Arena {
+    const int32_t* perm;   // clustered position -> source index
+    const int32_t* iperm;  // source index -> clustered position
+    const LowRankDesc* lr;
+    const DenseDesc* dd;
+    const uint8_t* comp_w;
+    const double* comp_s;
+    const ColTask* tasks;
+    const TaskRec* task_rec;
+    const uint8_t* qcodes;
+    const uint8_t* pcodes;
+    const double* dense;
+    const RowTile* tiles;
+    const TileDense* tdense;
+    const RowUnit* units;
+    const uint8_t* kp_info;
+    const SlotRec* slot_rec;
+    const TaskDest* task_dest;
+    const uint32_t* row_steps;
+    const double* comp_sl;  // s^P per component
+    const double* comp_sr;  // s^Q per component
+    const TcItem* tc_items;
+    const TcTask* tc_tasks;
+    const DenseUnit* dense_units;
+    const TcRowItem* tc_row_items;
+    const TcStep* tc_steps;
+};
+
+struct Work {
+    double* xc;        // [rhs][n]            x in clustered order (FP64)
+    int* xblk;         // [rhs][nblk]         largest exponent field of x per prep block
+    int* xe;           // [rhs]               largest exponent field of x
+    uint4* xq;         // [rhs][n_pad]        limbs of X (zero past n)
+    long long* lsplit; // [rhs][n_split*33][8] per-limb sums sum_i c_ij limb_l(X_i) of split tasks'
+                       //                     components (rows split_id*33 + j; zeroed by prep)
+    int* split_cnt;    // [rhs][n_split]      finished parts of each split task (zeroed by prep)
+    uint4* blimb;      // [rhs][n_slots]      row-side B rows: limbs of U (column by column)
+    long long* v;      // [n_comp][pv]        u in fixed point (tensor-memory kernels; the same memory)
+    uint4* part;       // [rhs][n_parts][128] 128-bit row sums of each row item (tensor-memory kernels)
+    uint4* plr;        // [rhs][n_tiles][kTileUnits][16] low-rank row sums of each row unit (128-bit)
+    double* pdense;    // [rhs][n_dslices][64] dense diagonal row sums per dense slice
+};
+
 namespace {
 
 // Fixed point: x (per rhs column) and u (per row tile) are held as integers
@@ -54,7 +98,7 @@ __device__ __forceinline__ long long comp_fixed(__int128 t, int shift, unsigned 
 }
 // U = V on a tile's coarser fixed point: round(V 2^-shift), shift in 0 .. 63.
 __device__ __forceinline__ long long tile_fixed(long long v, int shift) {
-    return (v + ((1ll << shift) >> 1)) >> shift;
+    return (v + (long long)((1ull << shift) >> 1)) >> shift;
 }
 
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
@@ -69,54 +113,19 @@ __device__ __forceinline__ uint32_t hsub2(uint32_t a, uint32_t b) {
 }
 
 // The eight limbs of X (|X| <= 2^62) as f16 values, limb k in half k:
-// X = sum_{k<7} l_k 2^(8k) + l_7 2^56 with l_0..l_6 in [0, 255] and l_7 in
-// [-64, 64].  The bytes of X + 2^62 are those limbs, the top one plus 64;
-// byte b becomes the f16 1024 + b (exponent bits 0x64 above it) and then the
-// integer b by one exact subtraction per pair.
+// X = sum_{k<7} l_k 2^(8k) + l_7 2^56 with l_0..l_6 in [-128, 127] and l_7 in
+// [-64, 64].  The bytes of X + 2^62 + 128 (1 + 2^8 + .. + 2^48) are those
+// limbs plus 128, the top one plus 64; byte b becomes the f16 1024 + b
+// (exponent bits 0x64 above it) and then the limb by one exact subtraction per
+// pair.
 __device__ __forceinline__ uint4 to_limbs(long long X) {
-    const unsigned long long Y = (unsigned long long)X + (1ull << 62);
+    const unsigned long long Y = (unsigned long long)X + 0x4080808080808080ull;
     const uint32_t lo = uint32_t(Y), hi = uint32_t(Y >> 32);
-    return make_uint4(hsub2(prmt(lo, 0x64646464u, 0x4140u), 0x64006400u),
-                      hsub2(prmt(lo, 0x64646464u, 0x4342u), 0x64006400u),
-                      hsub2(prmt(hi, 0x64646464u, 0x4140u), 0x64006400u),
-                      hsub2(prmt(hi, 0x64646464u, 0x4342u), 0x64406400u));
+    return make_uint4(hsub2(prmt(lo, 0x64646464u, 0x4140u), 0x64806480u),
+                      hsub2(prmt(lo, 0x64646464u, 0x4342u), 0x64806480u),
+                      hsub2(prmt(hi, 0x64646464u, 0x4140u), 0x64806480u),
+                      hsub2(prmt(hi, 0x64646464u, 0x4342u), 0x64406480u));
 }
-
-struct Arena {
-    const int32_t* perm;   // clustered position -> source index
-    const int32_t* iperm;  // source index -> clustered position
-    const LowRankDesc* lr;
-    const DenseDesc* dd;
-    const uint8_t* comp_w;
-    const double* comp_s;
-    const ColTask* tasks;
-    const TaskRec* task_rec;
-    const uint8_t* qcodes;
-    const uint8_t* pcodes;
-    const double* dense;
-    const RowTile* tiles;
-    const TileDense* tdense;
-    const RowUnit* units;
-    const uint8_t* kp_info;
-    const SlotRec* slot_rec;
-    const TaskDest* task_dest;
-    const uint32_t* row_steps;
-    const double* comp_sl;  // s^P per component
-    const double* comp_sr;  // s^Q per component
-};
-
-struct Work {
-    double* xc;        // [rhs][n]            x in clustered order (FP64)
-    int* xblk;         // [rhs][nblk]         largest exponent field of x per prep block
-    int* xe;           // [rhs]               largest exponent field of x
-    uint4* xq;         // [rhs][n_pad]        limbs of X (zero past n)
-    long long* lsplit; // [rhs][n_split*33][8] per-limb sums sum_i c_ij limb_l(X_i) of split tasks'
-                       //                     components (rows split_id*33 + j; zeroed by prep)
-    int* split_cnt;    // [rhs][n_split]      finished parts of each split task (zeroed by prep)
-    uint4* blimb;      // [rhs][n_slots]      row-side B rows: limbs of U
-    uint4* plr;        // [rhs][n_tiles][kTileUnits][16] low-rank row sums of each row unit (128-bit)
-    double* pdense;    // [rhs][n_dslices][64] dense diagonal row sums per dense slice
-};
 
 // -------------------------------------------------- bulk copies (TMA)
 
@@ -378,6 +387,28 @@ __device__ __forceinline__ __int128 ld_i128(const uint4* p) {
     const uint4 v = __ldcg(p);
     return (__int128)(((unsigned __int128)v.w << 96) | ((unsigned __int128)v.z << 64) |
                       ((unsigned __int128)v.y << 32) | v.x);
+}
+
+// A row k-pair's info byte: planes | nibble top plane << 3 | (top bits - 1) << 4.
+// Bytes of its digit groups, and the top plane's conversion constant.
+__device__ __forceinline__ int kp_bytes(int info) { return (info & 7) * 512 - ((info >> 3) & 1) * 256; }
+__device__ __forceinline__ uint32_t kp_hb(int info) { return (0x0400u | (1u << (info >> 4))) * 0x00010001u; }
+
+// Launch with programmatic stream serialization (the kernel may start while
+// its predecessor finishes; it waits in-kernel for the predecessor's results).
+template <typename... KArgs, typename... Args>
+cudaError_t launch_pdl(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k, static_cast<KArgs>(args)...);
 }
 
 }  // namespace

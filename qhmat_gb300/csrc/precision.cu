@@ -54,9 +54,12 @@
 #include "layout.hpp"
 #include "batch.hpp"
 #include "pf_layout.hpp"
+#include "tcgen05.hpp"
 
 namespace qhg {
 namespace pf {
+
+using namespace tc;
 
 // Warp roles of both kernels: warp 0 issues the copies, one thread of warp 1
 // the MMAs, warps 2 .. 2+C-1 convert, the last four drain tensor memory (lane
@@ -78,7 +81,6 @@ constexpr int kBStages = 2;
 constexpr int kNMax = 192;        // N of one pass (3 limbs x 64 right-hand sides)
 constexpr int kBTileBytes = kNMax * 128;   // B operand stage (N rows of 64 f16)
 constexpr int kURawBytes = kPfK * kPfMaxRhs * 4;  // 64 slots of FP32 u
-constexpr int kWaitLimit = 1 << 22;
 // K chunks one accumulation segment spans (a kernel template parameter, SEG,
 // chosen per handle: 2 by default, 1 for matrices whose tolerance asks for
 // it).  The tensor cores add each MMA's products into the FP32 accumulator
@@ -91,7 +93,6 @@ constexpr int kWaitLimit = 1 << 22;
 constexpr int kDefaultSegChunks = 2;
 constexpr int kAccStride = 256;
 constexpr int kStatusNonfinite = QH_STATUS_NONFINITE;
-constexpr int kStatusTimeout = QH_STATUS_TIMEOUT;
 
 // Shared-memory map (offsets from a 1024-byte-aligned base): the f16 A tiles
 // (16 KB each), the f16 B tiles (24 KB), the raw digit planes (8 KB) and, in
@@ -127,144 +128,6 @@ struct Work {
     float* ut;     // [n_slots][pu] u per row-side slot
     double* part;  // [n_parts][128][pu] FP64 partial sums of the row side
 };
-
-// ------------------------------------------------------------ primitives
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void mbar_expect(uint64_t* bar, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try(uint64_t* bar, unsigned parity) {
-    unsigned ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// Bounded wait; gives up when the block has been told to abort, or after
-// kWaitLimit tests (then it raises the abort flag and the timeout bit).
-__device__ __forceinline__ bool wait_bar(uint64_t* bar, unsigned parity, volatile int* abort_flag, int* status) {
-    for (int i = 0; i < kWaitLimit; ++i) {
-        if (mbar_try(bar, parity)) return true;
-        if ((i & 255) == 255 && *abort_flag) return false;
-    }
-    *abort_flag = 1;
-    if (status) atomicOr(status, kStatusTimeout);
-    return false;
-}
-// Pull a descriptor two items (chunks) ahead into L1, so that the roles that
-// read it find it there instead of waiting for L2 at every item.
-__device__ __forceinline__ void prefetch_l1(const void* ptr) {
-    asm volatile("prefetch.global.L1 [%0];" ::"l"(ptr));
-}
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_u32(dst)),
-                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
-}
-// 2-D tensor copy of the box at (x, y) of a tensor map into shared memory.
-__device__ __forceinline__ void tma_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-            smem_u32(dst)),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar))
-        : "memory");
-}
-
-// Tensor memory: allocate / free `cols` columns (one warp), the address
-// written to shared memory.
-__device__ __forceinline__ void tmem_alloc(uint32_t* dst, unsigned cols) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst)), "r"(cols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_free(uint32_t taddr, unsigned cols) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
-}
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-
-// Shared-memory matrix descriptor of a K-major operand in the 128-byte
-// swizzled layout: rows of 128 bytes, 8-row groups 1024 bytes apart (stride
-// byte offset), start advanced by 32 bytes per K step of 16 f16.
-__device__ __forceinline__ uint64_t sw128_desc(uint32_t addr) {
-    uint64_t d = 0;
-    d |= uint64_t((addr & 0x3FFFFu) >> 4);
-    d |= uint64_t(16 >> 4) << 16;    // leading byte offset (unused for swizzled K-major)
-    d |= uint64_t(1024 >> 4) << 32;  // stride byte offset
-    d |= uint64_t(1) << 46;          // descriptor version
-    d |= uint64_t(2) << 61;          // 128-byte swizzle
-    return d;
-}
-// Instruction descriptor: f16 x f16 -> f32, both K-major, M = 128, N.
-__host__ __device__ constexpr uint32_t mma_idesc(int n) {
-    return (1u << 4) | (uint32_t(n >> 3) << 17) | (uint32_t(128 >> 4) << 24);
-}
-__device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, int accumulate) {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
-        "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// Arrive on `bar` when every MMA this thread issued so far has completed.
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-                 : "memory");
-}
-// 16 consecutive FP32 columns of this warp's 32 tensor-memory lanes.
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
-    uint32_t r[16];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr)
-        : "memory");
-#pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-// Store 16 FP32 columns of this warp's 32 tensor-memory lanes.
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const float (&v)[16]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
-        "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])),
-        "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])),
-        "r"(__float_as_uint(v[8])), "r"(__float_as_uint(v[9])), "r"(__float_as_uint(v[10])), "r"(__float_as_uint(v[11])),
-        "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])), "r"(__float_as_uint(v[14])), "r"(__float_as_uint(v[15]))
-        : "memory");
-}
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
-__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
-    uint32_t r;
-    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
-    return r;
-}
-__device__ __forceinline__ uint32_t hsub2(uint32_t a, uint32_t b) {
-    uint32_t r;
-    asm("sub.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-    return r;
-}
-
-// Byte offset of 16-byte chunk c (elements 8c .. 8c+7) of row r in a 128-row
-// x 64-f16 tile, 128-byte swizzle.
-__device__ __forceinline__ uint32_t swz_chunk(int r, int c) {
-    return uint32_t((r >> 3) * 1024 + (r & 7) * 128 + ((c ^ (r & 7)) << 4));
-}
 
 // Eight digit bytes of plane m (top plane signed) -> eight f16 values
 // d 2^(E-25) for exponent field E: the f16 with exponent field E and mantissa

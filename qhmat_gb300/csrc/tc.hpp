@@ -1,0 +1,27 @@
+// Host interface of the tensor-memory kernels of the plain form (tc.cu).
+#pragma once
+
+#include "plain.hpp"
+
+namespace qhg {
+
+struct TcArgs {
+    Arena A;
+    Work W;
+    int n_items, n_row_items, n_dense, n_parts, n_tiles;
+    int rhs, pv, n, n_pad, n_split, n_dslices, sms;
+    double* y;
+    long long ld;
+    int* status;
+};
+
+// Right-hand-side columns the kernels take at once for an apply of rhs
+// columns (rows of V hold a multiple of it).
+int tc_columns(int rhs);
+// Once per device: the kernels' shared memory.
+cudaError_t tc_setup();
+// Column, row and combine kernels in stream order; mark(ctx, 2), if given, is
+// called after the column kernel.
+cudaError_t tc_launch(const TcArgs& a, cudaStream_t s, void (*mark)(void*, int), void* ctx);
+
+}  // namespace qhg
