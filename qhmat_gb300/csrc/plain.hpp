@@ -10,6 +10,7 @@
 
 #include "../../include/qhmat_gb300.h"
 #include "layout.hpp"
+#include "pdl.hpp"
 
 namespace qhg {
 
@@ -177,12 +178,6 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned b
         "l"(src), "r"(bytes), "r"(smem_u32(bar))
         : "memory");
 }
-
-// Programmatic dependent launch: a kernel lets its successor start early
-// (launch_dependents) and waits for its predecessor's results (wait) only
-// where it first reads them; without the launch attribute both are no-ops.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Status bits written by the kernels (status word of the apply).
 constexpr int kStatusNonfinite = QH_STATUS_NONFINITE;
@@ -393,23 +388,6 @@ __device__ __forceinline__ __int128 ld_i128(const uint4* p) {
 // Bytes of its digit groups, and the top plane's conversion constant.
 __device__ __forceinline__ int kp_bytes(int info) { return (info & 7) * 512 - ((info >> 3) & 1) * 256; }
 __device__ __forceinline__ uint32_t kp_hb(int info) { return (0x0400u | (1u << (info >> 4))) * 0x00010001u; }
-
-// Launch with programmatic stream serialization (the kernel may start while
-// its predecessor finishes; it waits in-kernel for the predecessor's results).
-template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k, static_cast<KArgs>(args)...);
-}
 
 }  // namespace
 }  // namespace qhg

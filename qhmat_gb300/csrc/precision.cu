@@ -52,6 +52,7 @@
 #include "../../include/qhmat_gb300.h"
 #include "errors.hpp"
 #include "layout.hpp"
+#include "pdl.hpp"
 #include "batch.hpp"
 #include "pf_layout.hpp"
 #include "tcgen05.hpp"
@@ -259,47 +260,110 @@ __device__ __forceinline__ void init_barriers(Shared& S, int astages, int conv_w
 
 // ------------------------------------------------------------ prep kernels
 
+// Both read x in 16-row blocks of 256 threads, a thread one column and every
+// (256 >> lw)-th row (columns in adjacent lanes: whole sectors of x's rows;
+// 2^lw >= p), so that each thread's loads are independent.
+constexpr int kPrepRows = 16;
+
 // Largest exponent field of each right-hand-side column (and the nonfinite
-// flag): block b, thread r reads rows 256b .. 256b+255 of column r.
-__global__ void __launch_bounds__(64) pf_xmax_kernel(const double* __restrict__ x, long long ld, int n, int p,
-                                                     int* ex, int* status) {
-    const int r = threadIdx.x;
-    if (r >= p) return;
+// flag).
+__global__ void __launch_bounds__(256) pf_xmax_kernel(const double* __restrict__ x, long long ld, int n, int p, int lw,
+                                                      int* ex, int* status) {
+    __shared__ int top[kPfMaxRhs];
+    pdl_trigger();
+    const int tid = threadIdx.x, r = tid & ((1 << lw) - 1);
+    if (tid < kPfMaxRhs) top[tid] = 0;
+    __syncthreads();
     int m = 0;
     bool bad = false;
-    const int i1 = min(n, (blockIdx.x + 1) * 256);
-    for (int i = blockIdx.x * 256; i < i1; ++i) {
-        const double v = x[(long long)i * ld + r];
-        const int e = int((__double_as_longlong(v) >> 52) & 0x7FF);
-        bad |= e == 0x7FF;
-        m = max(m, e == 0x7FF ? 0 : e);
+    if (r < p) {
+        const int i0 = int(blockIdx.x) * kPrepRows, i1 = min(n - i0, kPrepRows);
+        const double* src = x + (long long)i0 * ld + r;
+#pragma unroll 8
+        for (int i = tid >> lw; i < i1; i += 256 >> lw) {
+            const int e = int((__double_as_longlong(src[i * ld]) >> 52) & 0x7FF);
+            bad |= e == 0x7FF;
+            m = max(m, e == 0x7FF ? 0 : e);
+        }
+        atomicMax(top + r, m);
     }
     if (bad && status) atomicOr(status, kStatusNonfinite);
-    atomicMax(ex + r, m);
+    __syncthreads();
+    if (tid < p && top[tid]) atomicMax(ex + tid, top[tid]);
 }
 
-// XT[3r + l][i] = limb l of x'(perm[i], r) = x 2^(1037 - E_r); rows 3p .. N-1
-// and entries n .. n_ent-1 are zero.
-__global__ void __launch_bounds__(256) pf_xlimbs_kernel(const double* __restrict__ x, long long ld, int n, int p,
+// The f16 nearest to F 2^-38 (ties to even; a zero keeps `sign`), |F| < 2^53
+// with its last bit sticky: 24 leading bits, the last of them sticky, are an
+// exact FP32, which rounds to f16 as F 2^-38 itself does.
+__device__ __forceinline__ __half half_of(long long F, bool sign) {
+    const unsigned long long u = (unsigned long long)(F < 0 ? -F : F);
+    const int k = max(0, 40 - __clzll((long long)u));
+    const unsigned t = unsigned(u >> k) | ((u & ((1ull << k) - 1)) != 0);
+    const float f = float(int(t)) * __int_as_float((127 + k - 38) << 23);
+    return __float2half_rn((F < 0 || (F == 0 && sign)) ? -f : f);
+}
+// h 2^38 as an integer.
+__device__ __forceinline__ long long half_fixed(__half h) {
+    const unsigned b = __half_as_ushort(h), e = (b >> 10) & 31u;
+    const long long v = (long long)((b & 1023u) | (e ? 1024u : 0u)) << (e ? e + 13 : 14u);
+    return b & 0x8000u ? -v : v;
+}
+
+// XT[3r + l][i] = limb l of x'(perm[i], r) = x 2^(1037 - E_r), |x'| < 2^15; rows
+// 3p .. N-1 and entries n .. n_ent-1 are zero.
+//
+// Limb l is the f16 nearest to what the limbs before it leave.  In integers
+// (FP64 and its conversions run at a small fraction of the integer rate): the
+// limbs are multiples of 2^-24 and round at 2^-25 at the finest, so x' as an
+// integer times 2^-38 whose last bit is sticky gives the same limbs.  The tile
+// of 16 entries is turned in shared memory and stored as 32-byte runs.  With
+// the exponents, 8192 unknowns x 64 columns: 87 -> 21 us (one thread per
+// entry reading column by column, FP64 limbs).
+__global__ void __launch_bounds__(256) pf_xlimbs_kernel(const double* __restrict__ x, long long ld, int n, int p, int lw,
                                                         int n_ent, int N, const int32_t* __restrict__ perm,
-                                                        const int* __restrict__ ex, __half* __restrict__ xt) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_ent) return;
-    const long long src = i < n ? (long long)__ldg(perm + i) : -1;
-    for (int r = 0; r < p; ++r) {
-        const int E = ex[r];
-        double v = src >= 0 && E ? x[src * ld + r] : 0.0;
-        if (!isfinite(v)) v = 0.0;
-        v = scalbn(v, 1037 - E);
-        const __half a = __double2half(v);
-        const double r1 = v - double(__half2float(a));
-        const __half b = __double2half(r1);
-        const double r2 = r1 - double(__half2float(b));
-        xt[(long long)(3 * r) * n_ent + i] = a;
-        xt[(long long)(3 * r + 1) * n_ent + i] = b;
-        xt[(long long)(3 * r + 2) * n_ent + i] = __double2half(r2);
+                                                        const int* ex, __half* __restrict__ xt) {
+    constexpr int kPitch = kPrepRows + 2;  // halves: odd in words, so that columns fall into different banks
+    __shared__ __align__(4) __half tile[3 * kPfMaxRhs * kPitch];
+    pdl_trigger();
+    const int tid = threadIdx.x, r = tid & ((1 << lw) - 1), i0 = int(blockIdx.x) * kPrepRows;
+    pdl_wait();
+    if (r < p) {
+        const int E = __ldcg(ex + r);
+#pragma unroll 4
+        for (int i = tid >> lw; i < kPrepRows; i += 256 >> lw) {
+            unsigned long long bits = 0;
+            if (i0 + i < n) bits = (unsigned long long)__double_as_longlong(x[(long long)__ldg(perm + i0 + i) * ld + r]);
+            if ((~bits & 0x7FF0000000000000ull) == 0 || E == 0) bits = 0;  // (not finite: reported)
+            const int e = int(bits >> 52) & 0x7FF;
+            const bool sign = bits >> 63;
+            unsigned long long M = bits & 0xFFFFFFFFFFFFFull;
+            if (e) M |= 1ull << 52;
+            const int s = min(E - max(e, 1), 63);  // (E >= e of finite entries)
+            const long long V = (long long)(s > 0 ? (M >> s) | ((M & ((1ull << s) - 1)) != 0) : M);
+            const long long F = sign ? -V : V;
+            const __half a = half_of(F, sign);
+            const long long F1 = F - half_fixed(a);
+            const __half b = half_of(F1, false);
+            const __half c = half_of(F1 - half_fixed(b), false);
+            __half* t = tile + 3 * r * kPitch + i;
+            t[0] = a;
+            t[kPitch] = b;
+            t[2 * kPitch] = c;
+        }
     }
-    for (int row = 3 * p; row < N; ++row) xt[(long long)row * n_ent + i] = __ushort_as_half(0);
+    __syncthreads();
+    // runs of eight entries (n_ent is a multiple of eight)
+    const int runs = min(n_ent - i0, kPrepRows) / 8;
+    for (int k = tid; k < 2 * N; k += 256) {
+        const int row = k >> 1, q = k & 1;
+        if (q >= runs) continue;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (row < 3 * p) {
+            const auto* w = reinterpret_cast<const uint32_t*>(tile + row * kPitch + 8 * q);
+            v = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+        *reinterpret_cast<uint4*>(xt + (long long)row * n_ent + i0 + 8 * q) = v;
+    }
 }
 
 // ------------------------------------------------------------ column kernel
@@ -317,16 +381,18 @@ __global__ void __launch_bounds__(ColRoles::kThreads, 1) pf_column_kernel(Arena 
     __shared__ Shared S;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int it0 = __ldg(A.col_sched + blockIdx.x), it1 = __ldg(A.col_sched + blockIdx.x + 1);
+    pdl_trigger();
     if (tid == 0) {
         init_barriers(S, kAStages, kConvWarps);
         S.abort_flag = 0;
     }
+    if (warp == 1) tmem_alloc(&S.tmem, 512);
+    pdl_wait();
     if (tid < kPfMaxRhs) {
         const int E = tid < p ? W.ex[tid] : 0;
         S.ex[tid] = E;
         S.fxscale[tid] = E ? ldexpf(1.0f, max(-126, min(127, 24 + E - 1037))) : 0.0f;
     }
-    if (warp == 1) tmem_alloc(&S.tmem, 512);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -518,10 +584,21 @@ __global__ void __launch_bounds__(RowRoles::kThreads, 1) pf_row_kernel(Arena A, 
     __shared__ Shared S;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int it0 = __ldg(A.row_sched + blockIdx.x), it1 = __ldg(A.row_sched + blockIdx.x + 1);
+    pdl_trigger();
     if (tid == 0) {
         init_barriers(S, kAStages, kConvWarps);
         S.abort_flag = 0;
     }
+    if (warp == 1) tmem_alloc(&S.tmem, 512);
+    // B rows 3p .. N-1 of both f16 B stages stay zero (the converters write
+    // only rows < 3p; tensor copies of x write zeros there)
+    for (int idx = tid; idx < kBStages * (N - 3 * p) * 8; idx += RowRoles::kThreads) {
+        const int s = idx / ((N - 3 * p) * 8), rest = idx % ((N - 3 * p) * 8);
+        const int row = 3 * p + rest / 8, c = rest % 8;
+        *reinterpret_cast<uint4*>(sm + kOffBF16 + s * kBTileBytes + swz_chunk(row, c)) = make_uint4(0u, 0u, 0u, 0u);
+    }
+    fence_async_smem();
+    pdl_wait();
     if (tid < kPfMaxRhs) {
         const int E = tid < p ? W.ex[tid] : 0;
         S.ex[tid] = E;
@@ -531,15 +608,6 @@ __global__ void __launch_bounds__(RowRoles::kThreads, 1) pf_row_kernel(Arena A, 
         // smaller bound: k + (u_beta - the item's u_beta)
         S.ku[tid] = E ? 1037 - E - u_beta : kZeroColumn;
     }
-    // B rows 3p .. N-1 of both f16 B stages stay zero (the converters write
-    // only rows < 3p; tensor copies of x write zeros there)
-    for (int idx = tid; idx < kBStages * (N - 3 * p) * 8; idx += RowRoles::kThreads) {
-        const int s = idx / ((N - 3 * p) * 8), rest = idx % ((N - 3 * p) * 8);
-        const int row = 3 * p + rest / 8, c = rest % 8;
-        *reinterpret_cast<uint4*>(sm + kOffBF16 + s * kBTileBytes + swz_chunk(row, c)) = make_uint4(0u, 0u, 0u, 0u);
-    }
-    fence_async_smem();
-    if (warp == 1) tmem_alloc(&S.tmem, 512);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -777,19 +845,32 @@ __global__ void __launch_bounds__(256) pf_copy_kernel(const double* __restrict__
     for (; i < n; i += stride) dst[i] = src[i];
 }
 
-// y[perm[row] * ld + r] = the tile's partials, summed in K-split order.
+// y[perm[row] * ld + r] = the tile's partials, summed in K-split order.  Thread:
+// column r of a row (2^lw >= p columns; no divisions).
 __global__ void __launch_bounds__(256) pf_combine_kernel(const int32_t* __restrict__ perm,
                                                          const int32_t* __restrict__ tile_part0,
-                                                         const double* __restrict__ part, double* __restrict__ y,
-                                                         long long ld, int n, int p, int pu) {
-    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (long long)n * p) return;
-    const int row = int(idx / p), r = int(idx % p);
-    const int t = row / kPfM, j = row % kPfM;
+                                                         const double* part, double* __restrict__ y, long long ld, int n,
+                                                         int p, int lw, int pu) {
+    const int r = threadIdx.x & ((1 << lw) - 1);
+    const long long row = ((long long)blockIdx.x * 256 + threadIdx.x) >> lw;
+    pdl_wait();
+    if (r >= p || row >= n) return;
+    const int t = int(row / kPfM), j = int(row % kPfM);
     const int h0 = __ldg(tile_part0 + t), h1 = __ldg(tile_part0 + t + 1);
+    const double* src = part + ((long long)h0 * kPfM + j) * pu + r;
+    const long long stride = (long long)kPfM * pu;
+    const int dst = __ldg(perm + row);
     double s = 0.0;
-    for (int h = h0; h < h1; ++h) s += part[((long long)h * kPfM + j) * pu + r];
-    y[(long long)__ldg(perm + row) * ld + r] = s;
+    int h = h0;
+    for (; h + 4 <= h1; h += 4, src += 4 * stride) {
+        const double a = __ldcg(src), b = __ldcg(src + stride), c = __ldcg(src + 2 * stride), d = __ldcg(src + 3 * stride);
+        s += a;
+        s += b;
+        s += c;
+        s += d;
+    }
+    for (; h < h1; ++h, src += stride) s += __ldcg(src);
+    y[(long long)dst * ld + r] = s;
 }
 
 }  // namespace pf
@@ -919,28 +1000,28 @@ int pf_pass(const qh_pmatrix* m, const double* x, double* y, int p, long long ld
     cudaError_t e = cudaMemsetAsync(w + P.ex, 0, P.xt - P.ex, s);  // ex
     if (e != cudaSuccess) return cuda_err(e, "cudaMemsetAsync");
     mark(0);
-    pf::pf_xmax_kernel<<<(n + 255) / 256, 64, 0, s>>>(x, ld, n, p, W.ex, status);
-    pf::pf_xlimbs_kernel<<<(P.n_ent + 255) / 256, 256, 0, s>>>(x, ld, n, p, P.n_ent, P.N, m->A.perm, W.ex, W.xt);
+    // each kernel starts while its predecessor's last blocks finish and waits for
+    // them before it reads their results (8192 unknowns x 64 columns: 222 us kernel
+    // by kernel, 209 us as one pass)
+    int lw = 0;
+    while ((1 << lw) < p) ++lw;
+    pf::pf_xmax_kernel<<<(n + pf::kPrepRows - 1) / pf::kPrepRows, 256, 0, s>>>(x, ld, n, p, lw, W.ex, status);
+    e = launch_pdl(pf::pf_xlimbs_kernel, dim3(unsigned((P.n_ent + pf::kPrepRows - 1) / pf::kPrepRows)), dim3(256), 0, s, x,
+                   ld, n, p, lw, P.n_ent, P.N, m->A.perm, W.ex, W.xt);
     mark(1);
-    if (L.n_col_items > 0) {
-        if (m->seg == 1)
-            pf::pf_column_kernel<1><<<L.grid, pf::ColRoles::kThreads, pf::kSmemColumn, s>>>(m->A, W, map, p, P.N, P.pu,
-                                                                                           status);
-        else
-            pf::pf_column_kernel<2><<<L.grid, pf::ColRoles::kThreads, pf::kSmemColumn, s>>>(m->A, W, map, p, P.N, P.pu,
-                                                                                           status);
-    }
+    if (e == cudaSuccess && L.n_col_items > 0)
+        e = launch_pdl(m->seg == 1 ? pf::pf_column_kernel<1> : pf::pf_column_kernel<2>, dim3(unsigned(L.grid)),
+                       dim3(pf::ColRoles::kThreads), size_t(pf::kSmemColumn), s, m->A, W, map, p, P.N, P.pu, status);
     mark(2);
-    if (m->seg == 1)
-        pf::pf_row_kernel<1><<<L.grid, pf::RowRoles::kThreads, pf::kSmemRow, s>>>(m->A, W, map, p, P.N, P.pu, L.u_beta,
-                                                                                  status);
-    else
-        pf::pf_row_kernel<2><<<L.grid, pf::RowRoles::kThreads, pf::kSmemRow, s>>>(m->A, W, map, p, P.N, P.pu, L.u_beta,
-                                                                                  status);
+    if (e == cudaSuccess)
+        e = launch_pdl(m->seg == 1 ? pf::pf_row_kernel<1> : pf::pf_row_kernel<2>, dim3(unsigned(L.grid)),
+                       dim3(pf::RowRoles::kThreads), size_t(pf::kSmemRow), s, m->A, W, map, p, P.N, P.pu, L.u_beta,
+                       status);
     mark(3);
-    const long long total = (long long)n * p;
-    pf::pf_combine_kernel<<<unsigned((total + 255) / 256), 256, 0, s>>>(m->A.perm, m->tile_part0, W.part, y, ld, n,
-                                                                         p, P.pu);
+    if (e == cudaSuccess)
+        e = launch_pdl(pf::pf_combine_kernel, dim3(unsigned((((long long)n << lw) + 255) / 256)), dim3(256), 0, s,
+                       m->A.perm, m->tile_part0, W.part, y, ld, n, p, lw, P.pu);
+    if (e != cudaSuccess) return cuda_err(e, "CUDA kernel launch");
     mark(4);
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_err(e, "CUDA kernel launch");
