@@ -140,6 +140,14 @@ QH_API size_t qh_workspace_bytes(const qh_matrix* m, size_t rhs);
 QH_API int qh_matmul_device(const qh_matrix* m, const double* x, double* y, size_t rhs,
                      void* workspace, size_t workspace_bytes, void* stream, int* status);
 
+/* qh_matmul_device that waits for the result (the stream, on the host) and
+ * reports what its kernels flagged: QH_EINVAL "nonfinite right-hand side",
+ * QH_ERUNTIME "device copy wait timed out".  Nothing but the apply's kernels
+ * runs on the stream (the status word is a pinned int of the handle's).  Not
+ * for a stream that is being captured. */
+QH_API int qh_matmul_device_checked(const qh_matrix* m, const double* x, double* y, size_t rhs,
+                                    void* workspace, size_t workspace_bytes, void* stream);
+
 /* qh_matmul_device that also records four caller-created cudaEvent_t on
  * `stream`: before the right-hand-side preparation kernel, before the
  * column-side kernel, before the row-side kernel, and after it.  Profiling
@@ -268,6 +276,10 @@ QH_API size_t qh_pworkspace_bytes(const qh_pmatrix* m, size_t rhs);
  * Stream-ordered.  Column chunks of 64 right-hand sides run in turn. */
 QH_API int qh_pmatmul_device(const qh_pmatrix* m, const double* x, double* y, size_t rhs, void* workspace,
                              size_t workspace_bytes, void* stream, int* status);
+/* The same, waiting for the result and reporting the status, as
+ * qh_matmul_device_checked does. */
+QH_API int qh_pmatmul_device_checked(const qh_pmatrix* m, const double* x, double* y, size_t rhs, void* workspace,
+                                     size_t workspace_bytes, void* stream);
 /* The same, recording five caller-created cudaEvent_t around the first pass's
  * kernels: before the x preparation, before the column kernel, before the
  * row kernel, before the combine, after it.  Profiling aid. */

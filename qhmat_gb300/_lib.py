@@ -74,6 +74,8 @@ def load_library() -> C.CDLL:
     lib.qh_workspace_bytes.argtypes = [vp, sz]
     lib.qh_matmul_device.restype = i32
     lib.qh_matmul_device.argtypes = [vp, vp, vp, sz, vp, sz, vp, vp]
+    lib.qh_matmul_device_checked.restype = i32
+    lib.qh_matmul_device_checked.argtypes = [vp, vp, vp, sz, vp, sz, vp]
     lib.qh_matmul_device_profiled.restype = i32
     lib.qh_matmul_device_profiled.argtypes = [vp, vp, vp, sz, vp, sz, vp, vp, vp]
     lib.qh_matmul_device_static.restype = i32
@@ -102,6 +104,8 @@ def load_library() -> C.CDLL:
     lib.qh_pmatmul_host.argtypes = [vp, vp, vp, sz]
     lib.qh_pmatrix_host_direct.restype = i32
     lib.qh_pmatrix_host_direct.argtypes = [vp]
+    lib.qh_pmatmul_device_checked.restype = i32
+    lib.qh_pmatmul_device_checked.argtypes = [vp, vp, vp, sz, vp, sz, vp]
     lib.qh_pmatmul_device_profiled.restype = i32
     lib.qh_pmatmul_device_profiled.argtypes = [vp, vp, vp, sz, vp, sz, vp, vp, vp]
     ll = C.c_longlong

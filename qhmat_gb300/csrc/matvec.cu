@@ -59,6 +59,7 @@
 #include "batch.hpp"
 #include "errors.hpp"
 #include "layout.hpp"
+#include "status.hpp"
 #include "tc.hpp"
 
 namespace qhg {
@@ -1039,6 +1040,7 @@ struct qh_matrix {
     // warp_off[w] .. warp_off[w + 1] of the (reordered) task (unit) array
     int* sched = nullptr;
     int col_grid = 0, row_grid = 0;
+    StatusWords words;  // of qh_matmul_device_checked
     // lazily allocated scratch for calls without a workspace, and host staging
     std::mutex mu;
     void* own_ws = nullptr;  // qh_matmul_host's device buffer
@@ -1205,7 +1207,13 @@ int upload(Layout&& L, int device, qh_matrix** out) {
         delete m;
         return cuda_fail(e, "cudaMemcpy host-to-device");
     }
-    e = cudaFuncSetAttribute(row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowPipeSmem);
+    {
+        int* word = nullptr;  // the first status word (more only for calls at the same time)
+        e = m->words.take(&word);
+        if (e == cudaSuccess) m->words.give(word);
+    }
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowPipeSmem);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(column_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kColPipeSmem);
     if (e == cudaSuccess) e = tc_setup();
@@ -1594,6 +1602,20 @@ int qh_matmul_device_profiled(const qh_matrix* m, const double* x, double* y, si
         mm->dev_ws_bytes = need;
     }
     return launch(m, x, y, rhs, mm->dev_ws, static_cast<cudaStream_t>(stream), status, events4);
+}
+
+int qh_matmul_device_checked(const qh_matrix* m, const double* x, double* y, size_t rhs, void* workspace,
+                             size_t workspace_bytes, void* stream) {
+    if (!m) return fail(QH_EINVAL, "null matrix handle");
+    DeviceGuard g(m->device);
+    return checked_call(
+        const_cast<qh_matrix*>(m)->words, static_cast<cudaStream_t>(stream),
+        [&](int* word) { return qh_matmul_device(m, x, y, rhs, workspace, workspace_bytes, stream, word); },
+        [](cudaError_t e, int st) {
+            if (e != cudaSuccess) return cuda_fail(e, "CUDA kernel execution");
+            if (st & kStatusNonfinite) return fail(QH_EINVAL, "nonfinite right-hand side");
+            return fail(QH_ERUNTIME, "device copy wait timed out");
+        });
 }
 
 int qh_matmul_device_static(const qh_matrix* m, const double* x, double* y, size_t rhs, void* stream,

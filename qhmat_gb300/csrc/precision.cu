@@ -55,6 +55,7 @@
 #include "pdl.hpp"
 #include "batch.hpp"
 #include "pf_layout.hpp"
+#include "status.hpp"
 #include "tcgen05.hpp"
 
 namespace qhg {
@@ -887,6 +888,7 @@ struct qh_pmatrix {
     void* arena = nullptr;
     int32_t* tile_part0 = nullptr;
     pf::Arena A{};
+    StatusWords words;  // of qh_pmatmul_device_checked
     std::mutex mu;
     void* own_ws = nullptr;
     size_t own_ws_bytes = 0;
@@ -1074,6 +1076,15 @@ int pf_upload(const HostMatrix& hm, int device, int grid, double row_items_per_c
         delete m;
         return cuda_err(e, "precision form upload");
     }
+    {
+        int* word = nullptr;  // the first status word (more only for calls at the same time)
+        e = m->words.take(&word);
+        if (e != cudaSuccess) {
+            delete m;
+            return cuda_err(e, "cudaMallocHost");
+        }
+        m->words.give(word);
+    }
     std::vector<uint8_t>().swap(m->L.arena);
     const PfSections& S = m->L.sec;
     auto* b = static_cast<const uint8_t*>(m->arena);
@@ -1213,6 +1224,19 @@ int qh_pmatmul_device_profiled(const qh_pmatrix* m, const double* x, double* y, 
     return QH_OK;
 }
 
+int qh_pmatmul_device_checked(const qh_pmatrix* m, const double* x, double* y, size_t rhs, void* workspace,
+                              size_t workspace_bytes, void* stream) {
+    if (!m) return set_error(QH_EINVAL, "null matrix handle");
+    Guard g(m->device);
+    return checked_call(
+        const_cast<qh_pmatrix*>(m)->words, static_cast<cudaStream_t>(stream),
+        [&](int* word) { return qh_pmatmul_device(m, x, y, rhs, workspace, workspace_bytes, stream, word); },
+        [](cudaError_t e, int st) {
+            if (e != cudaSuccess) return cuda_err(e, "CUDA kernel execution");
+            if (st & QH_STATUS_NONFINITE) return set_error(QH_EINVAL, "nonfinite right-hand side");
+            return set_error(QH_ERUNTIME, "device copy wait timed out");
+        });
+}
 
 int qh_pmatmul_host(const qh_pmatrix* m, const double* x, double* y, size_t rhs) {
     if (!m) return set_error(QH_EINVAL, "null matrix handle");

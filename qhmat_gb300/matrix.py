@@ -21,7 +21,7 @@ from pathlib import Path
 
 import numpy as np
 
-from ._lib import QH_STATUS_NONFINITE, QH_STATUS_TIMEOUT, QhBlockDesc, QhPStats, QhStats, load_library, raise_for
+from ._lib import QhBlockDesc, QhPStats, QhStats, load_library, raise_for
 
 
 def _torch():
@@ -205,17 +205,12 @@ class HMatrix:
             workspace = torch.empty(need, dtype=torch.uint8, device=x.device)
         elif workspace.numel() * workspace.element_size() < need:
             raise ValueError("workspace too small")
-        status = torch.zeros(1, dtype=torch.int32, device=x.device)
         s = stream if stream is not None else torch.cuda.current_stream(x.device)
-        raise_for(self._lib.qh_matmul_device(self._h, x.data_ptr(), y.data_ptr(), rhs,
-                                             workspace.data_ptr(), need, s.cuda_stream,
-                                             status.data_ptr()))
+        args = (self._h, x.data_ptr(), y.data_ptr(), rhs, workspace.data_ptr(), need, s.cuda_stream)
         if check:
-            st = int(status.item())
-            if st & QH_STATUS_NONFINITE:
-                raise ValueError("nonfinite right-hand side")
-            if st & QH_STATUS_TIMEOUT:
-                raise RuntimeError("device copy wait timed out")
+            raise_for(self._lib.qh_matmul_device_checked(*args))
+        else:
+            raise_for(self._lib.qh_matmul_device(*args, None))
         return y
 
     def __matmul__(self, x):
@@ -350,16 +345,12 @@ class PrecisionHMatrix:
             workspace = torch.empty(need, dtype=torch.uint8, device=xt.device)
         elif workspace.numel() * workspace.element_size() < need:
             raise ValueError("workspace too small")
-        status = torch.zeros(1, dtype=torch.int32, device=xt.device)
         s = stream if stream is not None else torch.cuda.current_stream(xt.device)
-        raise_for(self._lib.qh_pmatmul_device(self._h, xt.data_ptr(), y.data_ptr(), rhs, workspace.data_ptr(),
-                                              need, s.cuda_stream, status.data_ptr()))
+        args = (self._h, xt.data_ptr(), y.data_ptr(), rhs, workspace.data_ptr(), need, s.cuda_stream)
         if check:
-            st = int(status.item())
-            if st & QH_STATUS_NONFINITE:
-                raise ValueError("nonfinite right-hand side")
-            if st & QH_STATUS_TIMEOUT:
-                raise RuntimeError("device copy wait timed out")
+            raise_for(self._lib.qh_pmatmul_device_checked(*args))
+        else:
+            raise_for(self._lib.qh_pmatmul_device(*args, None))
         return y
 
 
