@@ -51,6 +51,8 @@
 #include <queue>
 #include <type_traits>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 #include <unistd.h>
@@ -879,20 +881,31 @@ __global__ void __launch_bounds__(64) combine_kernel(Arena A, Work W, double* __
     y[(long long)out * ld + p] = d + lr;
 }
 
-// Validation: decode every code from the resident layout through the same
-// fragment routines the apply kernels feed to the MMA (group_digits uses the
-// permutes and masks of group_mma).  out[comp_base[c] + i] = code i of
-// component c (i: block column on the right side, clustered row on the left).
-__global__ void decode_col_kernel(Arena A, int n_tasks, const long long* __restrict__ comp_base, int* out) {
+// Decode every code from the resident layout through the same fragment
+// routines the apply kernels feed to the MMA (group_digits uses the permutes
+// and masks of group_mma).  out[comp_base[c] + i] = code i of component c
+// (i: block column on the right side, clustered row on the left), as it is or
+// as a factor entry (FP64, times the component's scale).
+__device__ __forceinline__ void put_code(int* out, long long i, long long code, const double*, int) {
+    out[i] = int(code);
+}
+__device__ __forceinline__ void put_code(double* out, long long i, long long code, const double* scale, int c) {
+    out[i] = __dmul_rn(double(code), scale[c]);
+}
+
+// Part y of gridDim.y: chunks of a task.
+template <class Out>
+__device__ __forceinline__ void decode_col(const Arena& A, int n_tasks, int block, int blocks,
+                                           const long long* __restrict__ comp_base, Out* out) {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int warps = gridDim.x * (blockDim.x >> 5);
-    for (int ti = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); ti < n_tasks; ti += warps) {
+    const int warps = blocks * (blockDim.x >> 5);
+    for (int ti = block * (blockDim.x >> 5) + (threadIdx.x >> 5); ti < n_tasks; ti += warps) {
         const ColTask T = A.tasks[ti];
         if (T.width == 0) continue;  // dense unit
         const int P = (T.width + 7) / 8;
         const bool nibtop = T.width - 8 * (P - 1) <= 4;
         const int RB = (P - 1) * 32 + (nibtop ? 16 : 32);
-        for (int ch = T.chunk0; ch < T.chunk0 + T.nchunks; ++ch) {
+        for (int ch = T.chunk0 + blockIdx.y; ch < T.chunk0 + T.nchunks; ch += gridDim.y) {
             const uint8_t* cb = A.qcodes + T.off + (long long)ch * T.stride;
             for (int q = 0; q < 2; ++q) {
                 const int rows = min(16, T.count - 16 * q);
@@ -913,7 +926,7 @@ __global__ void decode_col_kernel(Arena A, int n_tasks, const long long* __restr
                     const int c = A.task_rec[T.comp_idx + j].comp;
                     for (int k = 0; k < 8; ++k) {
                         const int i = ch * kColChunk + slot_entry(k >> 2, k & 3, t);
-                        if (i < T.n) out[comp_base[c] + i] = int(int64_t(u[hh][k]) - (int64_t(1) << (T.width - 1)));
+                        if (i < T.n) put_code(out, comp_base[c] + i, int64_t(u[hh][k]) - (int64_t(1) << (T.width - 1)), A.comp_sr, c);
                     }
                 }
             }
@@ -921,14 +934,24 @@ __global__ void decode_col_kernel(Arena A, int n_tasks, const long long* __restr
     }
 }
 
-__global__ void decode_row_kernel(Arena A, int n_units, const long long* __restrict__ comp_base, int* out) {
+// Part y of gridDim.y: a run of a unit's k-pairs (found by summing the bytes of
+// those before it).
+template <class Out>
+__device__ __forceinline__ void decode_row(const Arena& A, int n_units, int block, int blocks,
+                                           const long long* __restrict__ comp_base, Out* out) {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int warps = gridDim.x * (blockDim.x >> 5);
-    for (int ui = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); ui < n_units; ui += warps) {
+    const int warps = blocks * (blockDim.x >> 5);
+    for (int ui = block * (blockDim.x >> 5) + (threadIdx.x >> 5); ui < n_units; ui += warps) {
         const RowUnit U = A.units[ui];
         const RowTile T = A.tiles[U.tile];
-        const uint8_t* gp = A.pcodes + U.code_off;
-        for (int i = 0; i < U.nkps; ++i) {
+        const int per = (U.nkps + int(gridDim.y) - 1) / int(gridDim.y);
+        const int i0 = min(int(blockIdx.y) * per, U.nkps), i1 = min(i0 + per, U.nkps);
+        long long skip = 0;
+        for (int i = lane; i < i0; i += 32) skip += kp_bytes(A.kp_info[U.kp_off + U.h + i * U.H]);
+#pragma unroll
+        for (int o = 16; o; o >>= 1) skip += __shfl_xor_sync(0xFFFFFFFFu, skip, o);
+        const uint8_t* gp = A.pcodes + U.code_off + skip;
+        for (int i = i0; i < i1; ++i) {
             const int kp = U.h + i * U.H;
             const int info = A.kp_info[U.kp_off + kp];
             const int planes = info & 7, half = 1 << (info >> 4);
@@ -949,54 +972,120 @@ __global__ void decode_row_kernel(Arena A, int n_units, const long long* __restr
                     const int e = slot_entry(k >> 2, k & 3, t);
                     const int c = A.slot_rec[U.slot0 + 32 * i + e].comp;
                     if (c < 0) continue;
-                    out[comp_base[c] + T.row0 + tr] = int(u[hh][k]);
+                    put_code(out, comp_base[c] + T.row0 + tr, u[hh][k], A.comp_sl, c);
                 }
             }
         }
     }
 }
 
-// Dense reconstruction (src/qhmat/core.cpp:392-410): thread per entry of one
-// block (blocks by binary search over the entry prefix), value = the dense
-// entry or 0, plus, per component in order, (c^P s^P)(c^Q s^Q) with separate
-// IEEE multiplies and adds in the reference's order, written to
-// out[perm[row] * n + perm[col]].  Codes come from decode_*_kernel
-// (component-major: comp_base_l[c] + block row, comp_base_r[c] + block column).
-__global__ void reconstruct_kernel(Arena A, int n_lr, int n_dense, const long long* __restrict__ ent0,
-                                   long long total, const int* __restrict__ lcodes, const int* __restrict__ rcodes,
-                                   const long long* __restrict__ lbase, const long long* __restrict__ rbase,
-                                   int n, double* __restrict__ out) {
-    const int nb = n_lr + n_dense;
-    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
-         e += (long long)gridDim.x * blockDim.x) {
-        int lo = 0, hi = nb - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (ent0[mid] <= e) lo = mid;
-            else hi = mid - 1;
-        }
-        const long long le = e - ent0[lo];
-        double value = 0.0;
-        int row, col;
-        if (lo < n_lr) {
-            const LowRankDesc d = A.lr[lo];
-            const int i = int(le / d.n), k = int(le % d.n);
-            for (int j = 0; j < d.rank; ++j) {
-                const int c = d.comp0 + j;
-                const double l = __dmul_rn(double(lcodes[lbase[c] + i]), A.comp_sl[c]);
-                const double r = __dmul_rn(double(rcodes[rbase[c] + k]), A.comp_sr[c]);
-                value = __dadd_rn(value, __dmul_rn(l, r));
+// Blocks [0, col_blocks) of x decode the column side, the others the row side.
+template <class Out>
+__global__ void decode_kernel(Arena A, int n_tasks, int col_blocks, const long long* rbase, Out* rout, int n_units,
+                              const long long* lbase, Out* lout) {
+    if (int(blockIdx.x) < col_blocks) decode_col(A, n_tasks, blockIdx.x, col_blocks, rbase, rout);
+    else decode_row(A, n_units, int(blockIdx.x) - col_blocks, int(gridDim.x) - col_blocks, lbase, lout);
+}
+template <class Out>
+cudaError_t launch_decode(const Arena& A, int n_tasks, const long long* rbase, Out* rout, int n_units,
+                          const long long* lbase, Out* lout) {
+    const int cb = std::min((n_tasks + 7) / 8, 4096), rb = std::min((n_units + 7) / 8, 4096);
+    if (cb + rb == 0) return cudaSuccess;
+    decode_kernel<Out><<<dim3(unsigned(cb + rb), 8), 256>>>(A, n_tasks, cb, rbase, rout, n_units, lbase, lout);
+    return cudaGetLastError();
+}
+
+// A block of the matrix to reconstruct: its first tile, and where its factors
+// start (component-major: column j of P at left + j m).
+struct DenseOut {
+    long long tile0, left, right;
+};
+// Per component: where its entries start (decode_kernel's comp_base).
+__global__ void factor_base_kernel(Arena A, int n_lr, const DenseOut* blocks, long long* lbase, long long* rbase) {
+    const int b = blockIdx.x;
+    const LowRankDesc d = A.lr[b];
+    for (int j = threadIdx.x; j < d.rank; j += blockDim.x) {
+        lbase[d.comp0 + j] = blocks[b].left + (long long)j * d.m - d.row0;  // indexed by clustered row
+        rbase[d.comp0 + j] = blocks[b].right + (long long)j * d.n;
+    }
+}
+
+// Dense reconstruction (src/qhmat/core.cpp:392-410): value = the dense entry or
+// 0, plus, per component in order, (c^P s^P)(c^Q s^Q) with separate IEEE
+// multiplies and adds in the reference's order, written to
+// out[perm[row] * n + perm[col]].
+//
+// Bound by the FP64 unit: one multiply and one add per component and entry (the
+// factors are scaled once, by decode_kernel; scaling them per entry took six
+// operations).  One block per 32 x 32 tile, factors 16 components at a time in
+// shared memory, 2 x 4 entries a thread.  n = 2048, 2-D, 11587 components:
+// 657 -> 250 us (about 180 us by the rate of the FP64 unit).
+constexpr int kDenseTile = 32, kDenseComps = 16;
+__global__ void __launch_bounds__(128) reconstruct_kernel(Arena A, int n_lr, int nb, const DenseOut* __restrict__ blocks,
+                                                          const double* __restrict__ left,
+                                                          const double* __restrict__ right, int n,
+                                                          double* __restrict__ out) {
+    __shared__ double P[kDenseComps][kDenseTile], Q[kDenseComps][kDenseTile];
+    int lo = 0, hi = nb - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (blocks[mid].tile0 <= (long long)blockIdx.x) lo = mid;
+        else hi = mid - 1;
+    }
+    const DenseOut B = blocks[lo];
+    const int tile = int(blockIdx.x - B.tile0), tid = threadIdx.x;
+    LowRankDesc d = {};
+    long long off = 0;
+    if (lo < n_lr) {
+        d = A.lr[lo];
+    } else {
+        const DenseDesc e = A.dd[lo - n_lr];
+        d.row0 = e.row0, d.m = e.m, d.col0 = e.col0, d.n = e.n;
+        off = e.off;
+    }
+    const int tcols = (d.n + kDenseTile - 1) / kDenseTile;
+    const int i0 = tile / tcols * kDenseTile, k0 = tile % tcols * kDenseTile;
+    const int ti = tid >> 3, tk = tid & 7;  // rows ti, ti + 16; columns tk, tk + 8, ..
+    double v[2][4] = {};
+    if (lo < n_lr) {
+        const int tx = tid & 31, ty = tid >> 5;
+        for (int j0 = 0; j0 < d.rank; j0 += kDenseComps) {
+            const int jn = min(kDenseComps, d.rank - j0);
+            for (int j = ty; j < jn; j += 4) {
+                P[j][tx] = i0 + tx < d.m ? left[B.left + (long long)(j0 + j) * d.m + i0 + tx] : 0.0;
+                Q[j][tx] = k0 + tx < d.n ? right[B.right + (long long)(j0 + j) * d.n + k0 + tx] : 0.0;
             }
-            row = d.row0 + i;
-            col = d.col0 + k;
-        } else {
-            const DenseDesc d = A.dd[lo - n_lr];
-            const int i = int(le / d.n), k = int(le % d.n);
-            value = A.dense[d.off + (long long)k * d.m + i];
-            row = d.row0 + i;
-            col = d.col0 + k;
+            __syncthreads();
+            for (int j = 0; j < jn; ++j) {
+                const double a[2] = {P[j][ti], P[j][ti + 16]};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const double q = Q[j][tk + 8 * k];
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) v[i][k] = __dadd_rn(v[i][k], __dmul_rn(a[i], q));
+                }
+            }
+            __syncthreads();
         }
-        out[(long long)A.perm[row] * n + A.perm[col]] = value;
+    } else {
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int row = i0 + ti + 16 * i, col = k0 + tk + 8 * k;
+                if (row < d.m && col < d.n) v[i][k] = A.dense[off + (long long)col * d.m + row];
+            }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int row = i0 + ti + 16 * i;
+        if (row >= d.m) continue;
+        double* dst = out + (long long)A.perm[d.row0 + row] * n;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int col = k0 + tk + 8 * k;
+            if (col < d.n) dst[A.perm[d.col0 + col]] = v[i][k];
+        }
     }
 }
 
@@ -1041,6 +1130,8 @@ struct qh_matrix {
     int* sched = nullptr;
     int col_grid = 0, row_grid = 0;
     StatusWords words;  // of qh_matmul_device_checked
+    std::vector<LowRankDesc> lr;  // host copies of the blocks (reconstruct)
+    std::vector<DenseDesc> dd;
     // lazily allocated scratch for calls without a workspace, and host staging
     std::mutex mu;
     void* own_ws = nullptr;  // qh_matmul_host's device buffer
@@ -1220,6 +1311,13 @@ int upload(Layout&& L, int device, qh_matrix** out) {
     if (e != cudaSuccess) {
         delete m;
         return cuda_fail(e, "cudaFuncSetAttribute");
+    }
+    {
+        const auto* a = m->L.arena.data();
+        const auto* lr = reinterpret_cast<const LowRankDesc*>(a + m->L.sec.lr);
+        const auto* dd = reinterpret_cast<const DenseDesc*>(a + m->L.sec.dd);
+        m->lr.assign(lr, lr + m->L.n_lr);
+        m->dd.assign(dd, dd + m->L.n_dense);
     }
     // The host image is no longer needed once uploaded.
     std::vector<uint8_t>().swap(m->L.arena);
@@ -1440,6 +1538,44 @@ int check_rhs(const qh_matrix* m, size_t rhs) {
     if (m->L.order * rhs > size_t(INT32_MAX) * 256) return fail(QH_EOVERFLOW, "CUDA launch grid too large");
     return QH_OK;
 }
+
+}  // namespace
+
+namespace {
+
+// Makes the pages of a host buffer that is about to be written as a whole
+// present, on four threads (one write per page; the operating system clears the
+// page: a new 33 MB buffer took 1.1 ms on one thread, 0.41 ms on four, 0.53 ms
+// on eight, and 1.9 ms within a device-to-host copy).
+class PagePopulator {
+public:
+    PagePopulator(void* p, size_t bytes) {
+        if (!p || bytes < kPart) return;
+        const size_t n = std::min<size_t>({bytes / kPart, kThreads, std::max(1u, std::thread::hardware_concurrency())});
+        const size_t page = sysconf(_SC_PAGESIZE) > 0 ? size_t(sysconf(_SC_PAGESIZE)) : 4096;
+        auto* b = static_cast<uint8_t*>(p);
+        for (size_t k = 0; k < n; ++k)
+            try {
+                threads_[k] = std::thread([b, bytes, page, k, n] {
+                    const size_t at = bytes / n * k, end = k + 1 == n ? bytes : bytes / n * (k + 1);
+                    for (size_t i = at; i < end; i += page) *static_cast<volatile uint8_t*>(b + i) = 0;
+                    b[end - 1] = 0;  // (the buffer need not start on a page: a single absent
+                                     // page costs the copy 0.7 ms)
+                });
+            } catch (const std::system_error&) {
+                return;  // no more threads: the copy populates the rest
+            }
+    }
+    ~PagePopulator() { wait(); }
+    void wait() {
+        for (auto& t : threads_)
+            if (t.joinable()) t.join();
+    }
+
+private:
+    static constexpr size_t kThreads = 4, kPart = size_t(4) << 20;  // at least kPart bytes for a thread
+    std::thread threads_[kThreads];
+};
 
 }  // namespace
 
@@ -1782,78 +1918,60 @@ int qh_matrix_reconstruct(const qh_matrix* m, double* out, size_t out_count, int
     if (!out || out_count != n * n) return fail(QH_EINVAL, "output size does not match order * order");
     return guarded([&] {
         DeviceGuard g(m->device);
-        int rc = QH_OK;
-        const int n_lr = m->L.n_lr, n_dense = m->L.n_dense, nb = n_lr + n_dense;
-        std::vector<LowRankDesc> lr(static_cast<size_t>(n_lr));
-        std::vector<DenseDesc> dd(static_cast<size_t>(n_dense));
-        cudaError_t e = cudaSuccess;
-        if (n_lr) e = cudaMemcpy(lr.data(), m->A.lr, sizeof(LowRankDesc) * lr.size(), cudaMemcpyDeviceToHost);
-        if (e == cudaSuccess && n_dense)
-            e = cudaMemcpy(dd.data(), m->A.dd, sizeof(DenseDesc) * dd.size(), cudaMemcpyDeviceToHost);
-        if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpy device-to-host");
-        // code offsets (component-major, as qh_debug_decode lays them out) and
-        // the entry prefix of the blocks
-        std::vector<long long> lbase(size_t(m->L.n_comp) + 1, 0), rbase(size_t(m->L.n_comp) + 1, 0);
-        for (const auto& d : lr)
-            for (int j = 0; j < d.rank; ++j) {
-                lbase[size_t(d.comp0 + j) + 1] = d.m;
-                rbase[size_t(d.comp0 + j) + 1] = d.n;
-            }
-        for (size_t c = 0; c + 1 < lbase.size(); ++c) {
-            lbase[c + 1] += lbase[c];
-            rbase[c + 1] += rbase[c];
-        }
-        const long long ltotal = lbase.back(), rtotal = rbase.back();
-        std::vector<long long> lrow(lbase);  // left codes are indexed by clustered row
-        for (const auto& d : lr)
-            for (int j = 0; j < d.rank; ++j) lrow[size_t(d.comp0 + j)] -= d.row0;
-        std::vector<long long> ent0(size_t(nb) + 1, 0);
-        for (int b = 0; b < nb; ++b) {
-            const long long mm = b < n_lr ? lr[size_t(b)].m : dd[size_t(b - n_lr)].m;
-            const long long nn = b < n_lr ? lr[size_t(b)].n : dd[size_t(b - n_lr)].n;
-            ent0[size_t(b) + 1] = ent0[size_t(b)] + mm * nn;
-        }
-        const long long total = ent0[size_t(nb)];
-        // device scratch: codes, offsets, entry prefix, and the output if on the host
-        std::vector<void*> bufs;
-        auto alloc = [&](size_t bytes) -> void* {
-            void* p = nullptr;
-            if (cudaMalloc(&p, std::max<size_t>(bytes, 16)) != cudaSuccess) return nullptr;
-            bufs.push_back(p);
-            return p;
+        const int n_lr = m->L.n_lr, nb = n_lr + m->L.n_dense;
+        // blocks' tiles and factors (component-major)
+        std::vector<DenseOut> blocks(static_cast<size_t>(nb));
+        long long tiles = 0, ltotal = 0, rtotal = 0;
+        auto tiles_of = [](long long rows, long long cols) {
+            return ((rows + kDenseTile - 1) / kDenseTile) * ((cols + kDenseTile - 1) / kDenseTile);
         };
-        auto* d_lc = static_cast<int*>(alloc(4 * size_t(ltotal)));
-        auto* d_rc = static_cast<int*>(alloc(4 * size_t(rtotal)));
-        auto* d_lb = static_cast<long long*>(alloc(8 * lbase.size()));
-        auto* d_lr = static_cast<long long*>(alloc(8 * lbase.size()));
-        auto* d_rb = static_cast<long long*>(alloc(8 * rbase.size()));
-        auto* d_e0 = static_cast<long long*>(alloc(8 * ent0.size()));
-        double* d_out = out_on_device ? out : static_cast<double*>(alloc(8 * n * n));
-        if (!d_lc || !d_rc || !d_lb || !d_lr || !d_rb || !d_e0 || !d_out) {
-            for (void* p : bufs) cudaFree(p);
-            return fail(QH_ERUNTIME, "cudaMalloc: out of device memory");
+        for (int b = 0; b < nb; ++b) {
+            blocks[size_t(b)] = {tiles, ltotal, rtotal};
+            if (b < n_lr) {
+                const LowRankDesc& d = m->lr[size_t(b)];
+                ltotal += (long long)d.rank * d.m;
+                rtotal += (long long)d.rank * d.n;
+                tiles += tiles_of(d.m, d.n);
+            } else {
+                const DenseDesc& d = m->dd[size_t(b - n_lr)];
+                tiles += tiles_of(d.m, d.n);
+            }
         }
-        e = cudaMemcpy(d_lb, lbase.data(), 8 * lbase.size(), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemcpy(d_lr, lrow.data(), 8 * lrow.size(), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemcpy(d_rb, rbase.data(), 8 * rbase.size(), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemcpy(d_e0, ent0.data(), 8 * ent0.size(), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemset(d_out, 0, 8 * n * n);
-        if (e == cudaSuccess) {
-            if (m->L.n_tasks)
-                decode_col_kernel<<<std::max(1, std::min((m->L.n_tasks + 7) / 8, 4096)), 256>>>(m->A, m->L.n_tasks,
-                                                                                              d_rb, d_rc);
-            if (m->L.n_units)
-                decode_row_kernel<<<std::max(1, std::min((m->L.n_units + 7) / 8, 4096)), 256>>>(m->A, m->L.n_units,
-                                                                                              d_lr, d_lc);
-            if (total)
-                reconstruct_kernel<<<unsigned(std::min<long long>((total + 255) / 256, 65536)), 256>>>(
-                    m->A, n_lr, n_dense, d_e0, total, d_lc, d_rc, d_lb, d_rb, int(n), d_out);
+        if (tiles > INT32_MAX) return fail(QH_EOVERFLOW, "CUDA launch grid too large");
+        // one allocation: factors, bases, blocks, and the output if on the host
+        size_t bytes = 0;
+        auto take = [&](size_t b) {
+            const size_t o = bytes;
+            bytes += align256(std::max<size_t>(b, 1));
+            return o;
+        };
+        const size_t o_left = take(8 * size_t(ltotal)), o_right = take(8 * size_t(rtotal));
+        const size_t o_lb = take(8 * size_t(m->L.n_comp)), o_rb = take(8 * size_t(m->L.n_comp));
+        const size_t o_blocks = take(sizeof(DenseOut) * size_t(nb)), o_out = take(out_on_device ? 0 : 8 * n * n);
+        uint8_t* buf = nullptr;
+        if (cudaMalloc(&buf, bytes) != cudaSuccess) return fail(QH_ERUNTIME, "cudaMalloc: out of device memory");
+        auto* left = reinterpret_cast<double*>(buf + o_left);
+        auto* right = reinterpret_cast<double*>(buf + o_right);
+        auto* lb = reinterpret_cast<long long*>(buf + o_lb);
+        auto* rb = reinterpret_cast<long long*>(buf + o_rb);
+        auto* d_blocks = reinterpret_cast<DenseOut*>(buf + o_blocks);
+        double* d_out = out_on_device ? out : reinterpret_cast<double*>(buf + o_out);
+        cudaError_t e = cudaMemcpy(d_blocks, blocks.data(), sizeof(DenseOut) * blocks.size(), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess && n_lr) {
+            factor_base_kernel<<<unsigned(n_lr), 32>>>(m->A, n_lr, d_blocks, lb, rb);
+            e = launch_decode<double>(m->A, m->L.n_tasks, rb, right, m->L.n_units, lb, left);
+        }
+        if (e == cudaSuccess && tiles) {
+            reconstruct_kernel<<<unsigned(tiles), 128>>>(m->A, n_lr, nb, d_blocks, left, right, int(n), d_out);
             e = cudaGetLastError();
         }
-        if (e == cudaSuccess) e = cudaDeviceSynchronize();
-        if (e == cudaSuccess && !out_on_device) e = cudaMemcpy(out, d_out, 8 * n * n, cudaMemcpyDeviceToHost);
-        if (e != cudaSuccess) rc = cuda_fail(e, "reconstruct");
-        for (void* p : bufs) cudaFree(p);
+        // (host memory only; while the device works.  Before the allocation, its
+        // mappings and the page faults held each other up: 1.4 ms more.)
+        PagePopulator(out_on_device ? nullptr : out, 8 * n * n).wait();
+        if (e == cudaSuccess)
+            e = out_on_device ? cudaDeviceSynchronize() : cudaMemcpy(out, d_out, 8 * n * n, cudaMemcpyDeviceToHost);
+        const int rc = e == cudaSuccess ? QH_OK : cuda_fail(e, "reconstruct");
+        cudaFree(buf);
         return rc;
     });
 }
@@ -1896,11 +2014,8 @@ int qh_debug_decode(const qh_matrix* m, int side, int32_t* out, size_t out_count
         int rc = QH_OK;
         e = cudaMemcpy(d_off, off.data(), sizeof(long long) * off.size(), cudaMemcpyHostToDevice);
         if (e == cudaSuccess) {
-            if (side == 1)
-                decode_col_kernel<<<std::max(1, std::min((m->L.n_tasks + 7) / 8, 4096)), 256>>>(m->A, m->L.n_tasks, d_off, d_out);
-            else
-                decode_row_kernel<<<std::max(1, std::min((m->L.n_units + 7) / 8, 4096)), 256>>>(m->A, m->L.n_units, d_off, d_out);
-            e = cudaGetLastError();
+            e = launch_decode<int>(m->A, side == 1 ? m->L.n_tasks : 0, d_off, d_out, side == 0 ? m->L.n_units : 0, d_off,
+                                   d_out);
         }
         if (e == cudaSuccess) e = cudaMemcpy(out, d_out, sizeof(int) * total, cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) rc = cuda_fail(e, "debug decode");
