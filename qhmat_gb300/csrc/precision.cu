@@ -63,22 +63,30 @@ namespace pf {
 
 using namespace tc;
 
-// Warp roles of both kernels: warp 0 issues the copies, one thread of warp 1
-// the MMAs, warps 2 .. 2+C-1 convert, the last four drain tensor memory (lane
-// quarters 0..3).  The row kernel converts U as well as digit planes; it runs
-// eight converters (two per scheduler) and keeps its y sums in tensor memory,
-// which leaves them the registers.  The column kernel runs six.
-template <int CONV, int ASTAGES>
+// Warp roles of both kernels: warp 0 issues the copies, one elected thread of
+// warp 1 the MMAs; in the row kernel warps 2 .. 5 turn U into B tiles; two
+// groups of four warps convert digit planes, taking tiles in turn; the last
+// eight drain tensor memory (lane quarter = warp & 3), four for columns 0 .. 31,
+// four for 32 .. 63.
+//
+// What bounds both kernels is the time these roles take per small step (8192
+// unknowns x 64 columns: two or three planes an item on the column side, a
+// chunk of 64 slots on the row side), not memory or the MMAs.  With one group
+// of converters on every tile, four drain warps that loaded an item's
+// descriptors as they needed them, and descriptors built per MMA: column
+// kernel 69 us, row kernel 117; now 55 and 97.
+constexpr int kConvGroups = 2, kGroupWarps = 4;
+template <int UWARPS>
 struct Roles {
-    static constexpr int kConvWarps = CONV;
-    static constexpr int kEpiWarp0 = 2 + CONV;
-    static constexpr int kThreads = 32 * (kEpiWarp0 + 4);
-    static constexpr int kAStages = ASTAGES;  // digit-plane stages (raw and f16)
+    static constexpr int kUWarp0 = 2;
+    static constexpr int kConvWarp0 = 2 + UWARPS;
+    static constexpr int kEpiWarp0 = kConvWarp0 + kConvGroups * kGroupWarps;
+    static constexpr int kThreads = 32 * (kEpiWarp0 + 8);
+    static constexpr int kAStages = 4;  // digit-plane stages (raw and f16); even: a group sees every phase of its stages
 };
-using ColRoles = Roles<6, 4>;
-using RowRoles = Roles<8, 5>;
-constexpr int kConvWarp0 = 2;
-constexpr int kMaxAStages = 5;
+using ColRoles = Roles<0>;
+using RowRoles = Roles<4>;
+constexpr int kMaxAStages = 4;
 constexpr int kBStages = 2;
 constexpr int kNMax = 192;        // N of one pass (3 limbs x 64 right-hand sides)
 constexpr int kBTileBytes = kNMax * 128;   // B operand stage (N rows of 64 f16)
@@ -188,24 +196,25 @@ __device__ __forceinline__ uint32_t pack_h2(__half a, __half b) {
 // U of 64 slots (FP32, row stride pu) -> the f16 B tile: row 3r + l holds limb
 // l of u' = u 2^(ku[r] + dk) 256^(P-1) for the 64 slots of a chunk with P
 // planes (slots >= nvalid: 0; dk = the layout's u_beta minus the item's).
-// Pairs of slots are split with packed conversions.
-template <int NT>
-__device__ __forceinline__ void convert_u(const float* raw, uint8_t* tile, int p, int pu, int nvalid, int P,
-                                          const int* ku, int dk, int ctid) {
-    constexpr int kIters = (8 * kPfMaxRhs + NT - 1) / NT;
-#pragma unroll
-    for (int it = 0; it < kIters; ++it) {
-        const int idx = ctid + it * NT;
-        if (idx >= p * 8) break;
-        const int r = idx % p, kg = idx / p;
-        // 2^(ku + dk) 256^(P-1): the column's scale on this item's bound
-        const float sc = ku[r] == kZeroColumn ? 0.0f : pow2f_clamped(ku[r] + dk + 8 * (P - 1));
+// Pairs of slots are split with packed conversions.  Thread: one column, every
+// (NT >> lw)-th run of eight slots (2^lw >= p; a compile-time step for more
+// than 32 columns).
+template <int STEP>
+__device__ __forceinline__ void convert_u_runs(const float* raw, uint8_t* tile, int pu, int nvalid, float sc, int r,
+                                               int kg0, int step) {
+    const int n = STEP ? STEP : step;
+#pragma unroll(STEP ? 2 : 1)
+    for (int i = 0; i < (STEP ? 8 / (STEP ? STEP : 1) : 8); ++i) {
+        const int kg = kg0 + i * n;
+        if (!STEP && kg >= 8) break;
         float v[8];
+        const float* src = raw + 8 * kg * pu + r;
 #pragma unroll
-        for (int s = 0; s < 8; ++s) {
-            const int k = 8 * kg + s;
-            v[s] = k < nvalid ? raw[k * pu + r] * sc : 0.0f;
-        }
+        for (int s = 0; s < 8; ++s) v[s] = src[s * pu] * sc;
+        if (8 * kg + 8 > nvalid)
+#pragma unroll
+            for (int s = 0; s < 8; ++s)
+                if (8 * kg + s >= nvalid) v[s] = 0.0f;
         uint32_t h[3][4];
 #pragma unroll
         for (int s = 0; s < 8; s += 2) {
@@ -224,6 +233,16 @@ __device__ __forceinline__ void convert_u(const float* raw, uint8_t* tile, int p
             *reinterpret_cast<uint4*>(tile + swz_chunk(3 * r + l, kg)) = make_uint4(h[l][0], h[l][1], h[l][2], h[l][3]);
     }
 }
+template <int NT>
+__device__ __forceinline__ void convert_u(const float* raw, uint8_t* tile, int p, int lw, int pu, int nvalid, int P,
+                                          const int* ku, int dk, int ctid) {
+    const int r = ctid & ((1 << lw) - 1);
+    if (r >= p) return;
+    // 2^(ku + dk) 256^(P-1): the column's scale on this item's bound
+    const float sc = ku[r] == kZeroColumn ? 0.0f : pow2f_clamped(ku[r] + dk + 8 * (P - 1));
+    if (lw == 6) convert_u_runs<(NT >> 6)>(raw, tile, pu, nvalid, sc, r, ctid >> 6, 0);
+    else convert_u_runs<0>(raw, tile, pu, nvalid, sc, r, ctid >> lw, NT >> lw);
+}
 
 // Shared state of one block.
 struct Shared {
@@ -236,24 +255,24 @@ struct Shared {
     int ex[kPfMaxRhs];
     int ku[kPfMaxRhs];      // row kernel: U' = u 2^(ku + u_beta - item's u_beta); kZeroColumn for x = 0
     float fxscale[kPfMaxRhs];  // column kernel: 2^(24 + E_r - 1037)
-    float flitem[4][kPfMaxRhs];  // row kernel, per drain warp: the current item's 2^-(ku + ...) (low-rank sums)
+    float flitem[8][kPfMaxRhs / 2];  // row kernel, per drain warp: the current item's 2^-(ku + ...) (low-rank sums)
     float fdscale[kPfMaxRhs];  // row kernel: 2^(E_r - 1037) (dense sums, times 2^dense_exp)
 };
 
-__device__ __forceinline__ void init_barriers(Shared& S, int astages, int conv_warps) {
+__device__ __forceinline__ void init_barriers(Shared& S, int astages) {
     for (int i = 0; i < astages; ++i) {
         mbar_init(&S.a_full[i], 1);
-        mbar_init(&S.a_conv[i], conv_warps);
+        mbar_init(&S.a_conv[i], kGroupWarps);
         mbar_init(&S.a_empty[i], 1);
     }
     for (int i = 0; i < kBStages; ++i) {
         mbar_init(&S.b_full[i], 1);
-        mbar_init(&S.b_conv[i], conv_warps);
+        mbar_init(&S.b_conv[i], kGroupWarps);
         mbar_init(&S.b_empty[i], 1);
     }
     for (int i = 0; i < 2; ++i) {
         mbar_init(&S.acc_full[i], 1);
-        mbar_init(&S.acc_empty[i], 4);
+        mbar_init(&S.acc_empty[i], 8);
     }
     mbar_init(&S.drain, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -369,12 +388,29 @@ __global__ void __launch_bounds__(256) pf_xlimbs_kernel(const double* __restrict
 
 // ------------------------------------------------------------ column kernel
 
+// What a drain warp needs of a column item, and a component.
+struct ColTicket {
+    int nkc, count, comp0;
+};
+struct ColComp {
+    double scale;
+    int dest0, ndest;
+};
+__device__ __forceinline__ ColTicket load_ticket(const PfColItem* p) {
+    const uint4 a = ahead128(p), b = ahead128(reinterpret_cast<const uint4*>(p) + 1);
+    return ColTicket{int(a.w), int(b.y), int(b.z)};
+}
+__device__ __forceinline__ ColComp load_comp(const PfComp* p) {
+    const uint4 a = ahead128(p);
+    return ColComp{__hiloint2double(int(a.y), int(a.x)), int(a.z), int(a.w)};
+}
+
 // Persistent: block g runs column items col_sched[g] .. col_sched[g+1].
 template <int kSegChunks>
 __global__ void __launch_bounds__(ColRoles::kThreads, 1) pf_column_kernel(Arena A, Work W,
                                                                           const __grid_constant__ CUtensorMap xmap,
                                                                           int p, int N, int pu, int* status) {
-    constexpr int kConvWarps = ColRoles::kConvWarps, kEpiWarp0 = ColRoles::kEpiWarp0, kAStages = ColRoles::kAStages;
+    constexpr int kConvWarp0 = ColRoles::kConvWarp0, kEpiWarp0 = ColRoles::kEpiWarp0, kAStages = ColRoles::kAStages;
     constexpr int kOffAF16 = SmemMap<ColRoles>::kOffAF16, kOffBF16 = SmemMap<ColRoles>::kOffBF16,
                   kOffARaw = SmemMap<ColRoles>::kOffARaw;
     extern __shared__ uint8_t smem_dyn[];
@@ -384,7 +420,7 @@ __global__ void __launch_bounds__(ColRoles::kThreads, 1) pf_column_kernel(Arena 
     const int it0 = __ldg(A.col_sched + blockIdx.x), it1 = __ldg(A.col_sched + blockIdx.x + 1);
     pdl_trigger();
     if (tid == 0) {
-        init_barriers(S, kAStages, kConvWarps);
+        init_barriers(S, kAStages);
         S.abort_flag = 0;
     }
     if (warp == 1) tmem_alloc(&S.tmem, 512);
@@ -438,8 +474,9 @@ __global__ void __launch_bounds__(ColRoles::kThreads, 1) pf_column_kernel(Arena 
     } else if (warp == 1) {
         // ---- MMA issuer: per item, segments of kSegChunks K chunks, each into
         // the next of two accumulator buffers
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = mma_idesc(N);
+            const uint64_t a0 = sw128_desc(smem_u32(sm + kOffAF16)), b0 = sw128_desc(smem_u32(sm + kOffBF16));
             unsigned ai = 0, bi = 0, seg = 0;
             bool ok = true;
             for (int it = it0; it < it1 && ok; ++it) {
@@ -456,18 +493,17 @@ __global__ void __launch_bounds__(ColRoles::kThreads, 1) pf_column_kernel(Arena 
                         const int sb = bi % kBStages;
                         ok = wait_bar(&S.b_full[sb], (bi / kBStages) & 1, abort_flag, status);
                         if (!ok) break;
-                        const uint32_t b_addr = smem_u32(sm + kOffBF16 + sb * kBTileBytes);
+                        const uint64_t b = b0 + uint64_t(sb * (kBTileBytes >> 4));
                         for (int m = 0; m < I.planes; ++m) {
                             const int sa = ai % kAStages;
                             ok = wait_bar(&S.a_conv[sa], (ai / kAStages) & 1, abort_flag, status);
                             if (!ok) break;
                             tc_fence_after();
-                            const uint32_t a_addr = smem_u32(sm + kOffAF16 + sa * kPfTileBytes);
+                            const uint64_t a = a0 + uint64_t(sa * (kPfTileBytes >> 4));
+                            mma_f16(d, a, b, idesc, acc);
 #pragma unroll
-                            for (int ks = 0; ks < 4; ++ks) {
-                                mma_f16(d, sw128_desc(a_addr + 32 * ks), sw128_desc(b_addr + 32 * ks), idesc, acc);
-                                acc = 1;
-                            }
+                            for (int ks = 1; ks < 4; ++ks) mma_f16(d, a + 2 * ks, b + 2 * ks, idesc, 1);
+                            acc = 1;
                             mma_commit(&S.a_empty[sa]);
                             ++ai;
                         }
@@ -481,25 +517,27 @@ __global__ void __launch_bounds__(ColRoles::kThreads, 1) pf_column_kernel(Arena 
             mma_commit(&S.drain);
             for (int i = 0; i < kWaitLimit && !mbar_try(&S.drain, 0); ++i) {}
         }
+        __syncwarp();
     } else if (warp < kEpiWarp0) {
         // ---- converters: digit planes -> f16 A tiles
-        const int ctid = tid - kConvWarp0 * 32;
+        const unsigned group = unsigned(warp - kConvWarp0) / kGroupWarps;
+        const int ctid = (tid - kConvWarp0 * 32) % (kGroupWarps * 32);
         unsigned ai = 0;
         bool ok = true;
         for (int it = it0; it < it1 && ok; ++it) {
             const PfColItem I = A.col_items[it];
             if (it + 2 < it1) prefetch_l1(A.col_items + it + 2);
             for (int kc = 0; kc < I.nkc && ok; ++kc)
-                for (int m = 0; m < I.planes; ++m) {
+                for (int m = 0; m < I.planes; ++m, ++ai) {
+                    if (ai % kConvGroups != group) continue;
                     const int sa = ai % kAStages;
                     ok = wait_bar(&S.a_full[sa], (ai / kAStages) & 1, abort_flag, status);
                     if (!ok) break;
-                    convert_plane<kConvWarps * 32>(sm + kOffARaw + sa * kPfPlaneBytes, sm + kOffAF16 + sa * kPfTileBytes,
-                                                   m, I.planes, 0, 0, ctid);
+                    convert_plane<kGroupWarps * 32>(sm + kOffARaw + sa * kPfPlaneBytes, sm + kOffAF16 + sa * kPfTileBytes,
+                                                    m, I.planes, 0, 0, ctid);
                     fence_async_smem();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&S.a_conv[sa]);
-                    ++ai;
                 }
         }
     } else {
@@ -507,25 +545,38 @@ __global__ void __launch_bounds__(ColRoles::kThreads, 1) pf_column_kernel(Arena 
         // then u = s T 2^(24 + E_r - 1037) per component and column, in FP32
         // (u is stored as FP32; the FP64 pipe of this part would take ~20 us
         // per item for the same work)
-        const int q = warp & 3, j = 32 * q + lane;
+        const int q = warp & 3, j = 32 * q + lane, g0 = 2 * ((warp - kEpiWarp0) >> 2);
         unsigned seg = 0;
         bool ok = true;
+        // (item, component and slot are a chain of loads: the item is read two
+        // items ahead, its component one, the slot while the item's MMAs run)
+        ColTicket In, Inn;
+        ColComp Cn;
+        if (it0 < it1) {
+            In = load_ticket(A.col_items + it0);
+            Cn = load_comp(A.comps + In.comp0 + min(j, In.count - 1));
+            Inn = load_ticket(A.col_items + min(it0 + 1, it1 - 1));
+        }
         for (int it = it0; it < it1 && ok; ++it) {
-            const PfColItem I = A.col_items[it];
-            if (it + 2 < it1) prefetch_l1(A.col_items + it + 2);
-            PfComp C{};
-            if (j < I.count) C = A.comps[I.comp0 + j];
-            const float sf = float(C.scale);
-            float t[kPfMaxRhs];
+            const ColTicket I = In;
+            const ColComp C = Cn;
+            const bool on = j < I.count;
+            const uint32_t slot0 = ahead32(A.dests + (C.ndest ? C.dest0 : 0));
+            In = Inn;
+            Cn = load_comp(A.comps + In.comp0 + min(j, In.count - 1));
+            Inn = load_ticket(A.col_items + min(it + 2, it1 - 1));
+            const float sf = on ? float(C.scale) : 0.0f;
+            float t[32];
 #pragma unroll
-            for (int r = 0; r < kPfMaxRhs; ++r) t[r] = 0.0f;
+            for (int r = 0; r < 32; ++r) t[r] = 0.0f;
             for (int kc0 = 0; kc0 < I.nkc; kc0 += kSegChunks, ++seg) {
                 const int buf = seg & 1;
                 if (!(ok = wait_bar(&S.acc_full[buf], (seg >> 1) & 1, abort_flag, status))) break;
                 tc_fence_after();
                 const uint32_t base = tmem + (uint32_t(32 * q) << 16) + uint32_t(buf * kAccStride);
 #pragma unroll
-                for (int g = 0; g < kPfMaxRhs / 16; ++g) {
+                for (int h = 0; h < 2; ++h) {
+                    const int g = g0 + h;
                     if (16 * g >= p) break;
                     float v0[16], v1[16], v2[16];
                     tmem_ld16(base + 48 * g, v0);
@@ -539,7 +590,7 @@ __global__ void __launch_bounds__(ColRoles::kThreads, 1) pf_column_kernel(Arena 
                         const float a0 = c0 < 16 ? v0[c0] : (c0 < 32 ? v1[c0 - 16] : v2[c0 - 32]);
                         const float a1 = c1 < 16 ? v0[c1] : (c1 < 32 ? v1[c1 - 16] : v2[c1 - 32]);
                         const float a2 = c2 < 16 ? v0[c2] : (c2 < 32 ? v1[c2 - 16] : v2[c2 - 32]);
-                        t[16 * g + i] += (a0 + a1) + a2;
+                        t[16 * h + i] += (a0 + a1) + a2;
                     }
                 }
                 // accumulator drained: release it to the MMA warp
@@ -549,19 +600,21 @@ __global__ void __launch_bounds__(ColRoles::kThreads, 1) pf_column_kernel(Arena 
             }
             if (!ok) break;
 #pragma unroll
-            for (int g = 0; g < kPfMaxRhs / 16; ++g) {
+            for (int h = 0; h < 2; ++h) {
+                const int g = g0 + h;
                 if (16 * g >= p) break;
-                float u[16];
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
                     const int r = 16 * g + i;
-                    u[i] = (j < I.count && r < p) ? t[r] * sf * S.fxscale[r] : 0.0f;
+                    t[16 * h + i] = (on && r < p) ? t[16 * h + i] * sf * S.fxscale[r] : 0.0f;
                 }
-                for (int d = 0; d < (j < I.count ? C.ndest : 0); ++d) {
-                    const int slot = __ldg(A.dests + C.dest0 + d) & 0x0FFFFFFF;
-                    float4* dst = reinterpret_cast<float4*>(W.ut + (long long)slot * pu + 16 * g);
+                for (int d = 0; d < (on ? C.ndest : 0); ++d) {
+                    const uint32_t dest = d == 0 ? slot0 : uint32_t(__ldg(A.dests + C.dest0 + d));
+                    float4* dst = reinterpret_cast<float4*>(W.ut + (long long)int(dest & 0x0FFFFFFFu) * pu + 16 * g);
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) dst[k] = make_float4(u[4 * k], u[4 * k + 1], u[4 * k + 2], u[4 * k + 3]);
+                    for (int k = 0; k < 4; ++k)
+                        dst[k] = make_float4(t[16 * h + 4 * k], t[16 * h + 4 * k + 1], t[16 * h + 4 * k + 2],
+                                             t[16 * h + 4 * k + 3]);
                 }
             }
         }
@@ -577,7 +630,7 @@ template <int kSegChunks>
 __global__ void __launch_bounds__(RowRoles::kThreads, 1) pf_row_kernel(Arena A, Work W,
                                                                        const __grid_constant__ CUtensorMap xmap, int p,
                                                                        int N, int pu, int u_beta, int* status) {
-    constexpr int kConvWarps = RowRoles::kConvWarps, kEpiWarp0 = RowRoles::kEpiWarp0, kAStages = RowRoles::kAStages;
+    constexpr int kConvWarp0 = RowRoles::kConvWarp0, kEpiWarp0 = RowRoles::kEpiWarp0, kAStages = RowRoles::kAStages;
     constexpr int kOffAF16 = SmemMap<RowRoles>::kOffAF16, kOffBF16 = SmemMap<RowRoles>::kOffBF16,
                   kOffARaw = SmemMap<RowRoles>::kOffARaw, kOffBRaw = SmemMap<RowRoles>::kOffBRaw;
     extern __shared__ uint8_t smem_dyn[];
@@ -587,7 +640,7 @@ __global__ void __launch_bounds__(RowRoles::kThreads, 1) pf_row_kernel(Arena A, 
     const int it0 = __ldg(A.row_sched + blockIdx.x), it1 = __ldg(A.row_sched + blockIdx.x + 1);
     pdl_trigger();
     if (tid == 0) {
-        init_barriers(S, kAStages, kConvWarps);
+        init_barriers(S, kAStages);
         S.abort_flag = 0;
     }
     if (warp == 1) tmem_alloc(&S.tmem, 512);
@@ -659,8 +712,9 @@ __global__ void __launch_bounds__(RowRoles::kThreads, 1) pf_row_kernel(Arena A, 
     } else if (warp == 1) {
         // ---- MMA issuer: per item, segments of up to kSegChunks chunks of one
         // kind (low rank or dense), each into the next of two buffers
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = mma_idesc(N);
+            const uint64_t a0 = sw128_desc(smem_u32(sm + kOffAF16)), b0 = sw128_desc(smem_u32(sm + kOffBF16));
             unsigned ai = 0, bi = 0, seg = 0;
             bool ok = true;
             for (int it = it0; it < it1 && ok; ++it) {
@@ -683,19 +737,18 @@ __global__ void __launch_bounds__(RowRoles::kThreads, 1) pf_row_kernel(Arena A, 
                         const int sb = bi % kBStages;
                         ok = wait_bar(&S.b_conv[sb], (bi / kBStages) & 1, abort_flag, status);
                         if (!ok) break;
-                        const uint32_t b_addr = smem_u32(sm + kOffBF16 + sb * kBTileBytes);
+                        const uint64_t b = b0 + uint64_t(sb * (kBTileBytes >> 4));
                         const int nt = C.kind == 0 ? C.planes : 3;
                         for (int m = 0; m < nt; ++m) {
                             const int sa = ai % kAStages;
                             ok = wait_bar(&S.a_conv[sa], (ai / kAStages) & 1, abort_flag, status);
                             if (!ok) break;
                             tc_fence_after();
-                            const uint32_t a_addr = smem_u32(sm + kOffAF16 + sa * kPfTileBytes);
+                            const uint64_t a = a0 + uint64_t(sa * (kPfTileBytes >> 4));
+                            mma_f16(d, a, b, idesc, acc);
 #pragma unroll
-                            for (int ks = 0; ks < 4; ++ks) {
-                                mma_f16(d, sw128_desc(a_addr + 32 * ks), sw128_desc(b_addr + 32 * ks), idesc, acc);
-                                acc = 1;
-                            }
+                            for (int ks = 1; ks < 4; ++ks) mma_f16(d, a + 2 * ks, b + 2 * ks, idesc, 1);
+                            acc = 1;
                             mma_commit(&S.a_empty[sa]);
                             ++ai;
                         }
@@ -709,9 +762,12 @@ __global__ void __launch_bounds__(RowRoles::kThreads, 1) pf_row_kernel(Arena A, 
             mma_commit(&S.drain);
             for (int i = 0; i < kWaitLimit && !mbar_try(&S.drain, 0); ++i) {}
         }
-    } else if (warp < kEpiWarp0) {
-        const int ctid = tid - kConvWarp0 * 32;
-        unsigned ai = 0, bi = 0;
+        __syncwarp();
+    } else if (warp < kConvWarp0) {
+        // ---- U converters: each chunk's B tile
+        const int ctid = tid - RowRoles::kUWarp0 * 32;
+        const int lw = p > 1 ? 32 - __clz(p - 1) : 0;
+        unsigned bi = 0;
         bool ok = true;
         for (int it = it0; it < it1 && ok; ++it) {
             const PfRowItem I = A.row_items[it];
@@ -722,26 +778,42 @@ __global__ void __launch_bounds__(RowRoles::kThreads, 1) pf_row_kernel(Arena A, 
                 ok = wait_bar(&S.b_full[sb], (bi / kBStages) & 1, abort_flag, status);
                 if (!ok) break;
                 if (C.kind == 0)
-                    convert_u<kConvWarps * 32>(reinterpret_cast<const float*>(sm + kOffBRaw + sb * kURawBytes),
-                                               sm + kOffBF16 + sb * kBTileBytes, p, pu, C.nvalid, C.planes, S.ku,
+                    convert_u<kGroupWarps * 32>(reinterpret_cast<const float*>(sm + kOffBRaw + sb * kURawBytes),
+                                               sm + kOffBF16 + sb * kBTileBytes, p, lw, pu, C.nvalid, C.planes, S.ku,
                                                u_beta - I.u_beta, ctid);
                 fence_async_smem();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&S.b_conv[sb]);
                 ++bi;
+            }
+        }
+    } else if (warp < kEpiWarp0) {
+        // ---- converters: digit planes -> f16 A tiles (dense limb tiles pass)
+        const unsigned group = unsigned(warp - kConvWarp0) / kGroupWarps;
+        const int ctid = (tid - kConvWarp0 * 32) % (kGroupWarps * 32);
+        unsigned ai = 0;
+        bool ok = true;
+        for (int it = it0; it < it1 && ok; ++it) {
+            const PfRowItem I = A.row_items[it];
+            for (int c = 0; c < I.nchunks && ok; ++c) {
+                const PfRowChunk C = A.chunks[I.chunk0 + c];
+                if (c + 2 < I.nchunks) prefetch_l1(A.chunks + I.chunk0 + c + 2);
                 const int nt = C.kind == 0 ? C.planes : 3;
-                for (int m = 0; m < nt; ++m) {
+                for (int m = 0; m < nt; ++m, ++ai) {
+                    if (ai % kConvGroups != group) continue;
                     const int sa = ai % kAStages;
                     ok = wait_bar(&S.a_full[sa], (ai / kAStages) & 1, abort_flag, status);
                     if (!ok) break;
-                    if (C.kind == 0)
-                        convert_plane<kConvWarps * 32>(sm + kOffARaw + sa * kPfPlaneBytes,
-                                                       sm + kOffAF16 + sa * kPfTileBytes, m, C.planes,
-                                                       24 - 8 * (C.planes - 1), C.half, ctid);
+                    if (C.kind == 0) {
+                        const uint8_t* raw = sm + kOffARaw + sa * kPfPlaneBytes;
+                        uint8_t* tile = sm + kOffAF16 + sa * kPfTileBytes;
+                        const int P = C.planes, ebias = 24 - 8 * (P - 1);
+                        if (C.half == 0) convert_plane<kGroupWarps * 32>(raw, tile, m, P, ebias, 0, ctid);
+                        else convert_plane<kGroupWarps * 32>(raw, tile, m, P, ebias, C.half, ctid);
+                    }
                     fence_async_smem();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&S.a_conv[sa]);
-                    ++ai;
                 }
             }
         }
@@ -751,7 +823,8 @@ __global__ void __launch_bounds__(RowRoles::kThreads, 1) pf_row_kernel(Arena A, 
         // tensor memory (columns 192..255, which no MMA writes: N <= 192 and
         // the second accumulator starts at 256); the item's partial y stored
         // in FP64
-        const int q = warp & 3, j = 32 * q + lane;
+        const int q = warp & 3, j = 32 * q + lane, g0 = 2 * ((warp - kEpiWarp0) >> 2);
+        float* const flitem = S.flitem[warp - kEpiWarp0];  // of columns 16 g0 ..
         const uint32_t yb = tmem + (uint32_t(32 * q) << 16) + 192u;
         unsigned seg = 0;
         bool ok = true;
@@ -762,12 +835,13 @@ __global__ void __launch_bounds__(RowRoles::kThreads, 1) pf_row_kernel(Arena A, 
 #pragma unroll
                 for (int i = 0; i < 16; ++i) z[i] = 0.0f;
 #pragma unroll
-                for (int g = 0; g < kPfMaxRhs / 16; ++g)
+                for (int g = g0; g < g0 + 2; ++g)
                     if (16 * g < p) tmem_st16(yb + 16 * g, z);
                 tmem_wait_st();
                 // this item's low-rank scales 2^-(ku + u_beta - item's u_beta)
-                for (int r = lane; r < kPfMaxRhs; r += 32)
-                    S.flitem[q][r] = S.ku[r] == kZeroColumn ? 0.0f : pow2f_clamped(-(S.ku[r] + u_beta - I.u_beta));
+                const int ku = S.ku[16 * g0 + lane];
+                __syncwarp();
+                flitem[lane] = ku == kZeroColumn ? 0.0f : pow2f_clamped(-(ku + u_beta - I.u_beta));
                 __syncwarp();
             }
             const float dexp = ldexpf(1.0f, max(-126, min(127, I.dense_exp)));
@@ -783,7 +857,7 @@ __global__ void __launch_bounds__(RowRoles::kThreads, 1) pf_row_kernel(Arena A, 
                 tc_fence_after();
                 const uint32_t base = tmem + (uint32_t(32 * q) << 16) + uint32_t(buf * kAccStride);
 #pragma unroll 1
-                for (int g = 0; g < kPfMaxRhs / 16; ++g) {
+                for (int g = g0; g < g0 + 2; ++g) {
                     if (16 * g >= p) break;
                     float v0[16], v1[16], v2[16], y[16];
                     tmem_ld16(base + 48 * g, v0);
@@ -798,7 +872,7 @@ __global__ void __launch_bounds__(RowRoles::kThreads, 1) pf_row_kernel(Arena A, 
                         const float a0 = c0 < 16 ? v0[c0] : (c0 < 32 ? v1[c0 - 16] : v2[c0 - 32]);
                         const float a1 = c1 < 16 ? v0[c1] : (c1 < 32 ? v1[c1 - 16] : v2[c1 - 32]);
                         const float a2 = c2 < 16 ? v0[c2] : (c2 < 32 ? v1[c2 - 16] : v2[c2 - 32]);
-                        const float sc = kind == 0 ? S.flitem[q][r] : S.fdscale[r] * dexp;
+                        const float sc = kind == 0 ? flitem[r - 16 * g0] : S.fdscale[r] * dexp;
                         y[i] = fmaf((a0 + a1) + a2, sc, y[i]);
                     }
                     tmem_st16(yb + 16 * g, y);
@@ -811,7 +885,7 @@ __global__ void __launch_bounds__(RowRoles::kThreads, 1) pf_row_kernel(Arena A, 
             if (!ok) break;
             double* out = W.part + ((long long)I.part * kPfM + j) * pu;
 #pragma unroll 1
-            for (int g = 0; g < kPfMaxRhs / 16; ++g) {
+            for (int g = g0; g < g0 + 2; ++g) {
                 if (16 * g >= p) break;
                 float y[16];
                 tmem_ld16(yb + 16 * g, y);

@@ -173,32 +173,6 @@ __device__ __forceinline__ uint64_t limb_desc(uint32_t addr, uint32_t col) {
     return d;
 }
 
-// Loads of read-only descriptors ahead of their use.  Volatile: plain __ldg is
-// free to sink to the use, which puts an L2 round trip into every step.  They
-// are also issued unconditionally (from some descriptor that exists): a load
-// under a condition is followed by a copy that waits for it.
-__device__ __forceinline__ uint4 ahead128(const void* p) {
-    uint4 v;
-    asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ uint2 ahead64(const void* p) {
-    uint2 v;
-    asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ uint32_t ahead32(const void* p) {
-    uint32_t v;
-    asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));
-    return v;
-}
-
-// True on one lane of a converged warp.
-__device__ __forceinline__ bool elect_one() {
-    uint32_t p;
-    asm volatile("{\n .reg .pred e;\n elect.sync _|e, 0xffffffff;\n selp.u32 %0, 1, 0, e;\n}" : "=r"(p));
-    return p != 0;
-}
 __device__ __forceinline__ void mma_add(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc) {
     asm volatile(
         "{\n .reg .pred p;\n setp.eq.b32 p, 0, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d),

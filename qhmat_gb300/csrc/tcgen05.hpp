@@ -99,6 +99,32 @@ __device__ __forceinline__ uint64_t sw128_desc(uint32_t addr) {
     d |= uint64_t(2) << 61;          // 128-byte swizzle
     return d;
 }
+// Loads of read-only descriptors ahead of their use.  Volatile: plain __ldg is
+// free to sink to the use, which puts an L2 round trip into every step.  They
+// are also issued unconditionally (from some descriptor that exists): a load
+// under a condition is followed by a copy that waits for it.
+__device__ __forceinline__ uint4 ahead128(const void* p) {
+    uint4 v;
+    asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint2 ahead64(const void* p) {
+    uint2 v;
+    asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint32_t ahead32(const void* p) {
+    uint32_t v;
+    asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+
+// True on one lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n .reg .pred e;\n elect.sync _|e, 0xffffffff;\n selp.u32 %0, 1, 0, e;\n}" : "=r"(p));
+    return p != 0;
+}
 // Instruction descriptor: f16 x f16 -> f32, both K-major, M = 128, N.
 __host__ __device__ constexpr uint32_t mma_idesc(int n) {
     return (1u << 4) | (uint32_t(n >> 3) << 17) | (uint32_t(128 >> 4) << 24);
