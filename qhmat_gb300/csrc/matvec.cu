@@ -1376,7 +1376,7 @@ size_t rhs_chunk(size_t rhs) { return std::min(rhs, kMaxRhsChunk); }
 
 struct WsPlan {
     size_t xc, xblk, xe, xq, lsplit, cnt, blimb, part, plr, pdense, total, zero0, zero_bytes;
-    int nblk, pv;  // pv > 0: columns of a row of V (the tensor-memory kernels)
+    int nblk, pv;  // pv > 0: columns of a row of V, an even number (the tensor-memory kernels)
 };
 
 // x limbs are read by whole 32-entry chunks: pad past the last chunk.
@@ -1401,8 +1401,7 @@ WsPlan ws_plan(const Layout& L, size_t rhs, bool tc) {
     w.xc = take(8 * L.order * rhs);
     w.xq = take(16 * padded_order(L) * rhs);
     if (tc) {  // V and the row items' sums
-        const int R = tc_columns(int(rhs));
-        w.pv = (int(rhs) + R - 1) / R * R;
+        w.pv = (int(rhs) + 1) & ~1;
         w.blimb = take(8 * size_t(L.n_comp) * size_t(w.pv));
         w.part = take(16 * 128 * size_t(L.n_parts) * rhs);
     } else {  // B rows and row sums of the column-by-column kernels

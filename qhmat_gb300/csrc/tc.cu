@@ -22,10 +22,11 @@
 // 0.8 per digit, once per R columns), V -> limbs, and the 64-bit fold of the
 // sums; per step of two A tiles a handshake of each role.  Measured against
 // the column-by-column kernels (device us): 16384 unknowns x 16 columns 556 ->
-// 186, 8192 (3-D) x 64 columns 2654 -> 598, 2048 x 4 43 -> 28.  Tried and
+// 186, 8192 (3-D) x 64 columns 2654 -> 565, 2048 x 4 43 -> 28.  Tried and
 // slower: one handshake per A tile (782 at 64 columns), register prefetch of V
-// instead of asynchronous copies, three stages, B operands of 16 columns
-// (shared memory), waiting warps that sleep or wait on a leader.
+// instead of asynchronous copies, three stages, waiting warps that sleep or
+// wait on a leader.  B operands of 16 columns in the column kernel gave 3 % at
+// 16 and 64 columns and lost 6 % at 24: the drains' work goes with the columns.
 //
 // Sums: an accumulator takes at most 128 entries, each product below 2^15 in
 // magnitude times 2^-24, so it is an integer below 2^22 times 2^-24, exact (the
@@ -260,6 +261,35 @@ __device__ __forceinline__ __int128 join_limbs(const unsigned long long (&v)[4],
     return (__int128)(long long)(v[0] - b) + ((__int128)(long long)(v[1] - b) << 16) +
            ((__int128)(long long)(v[2] - b) << 32) + ((__int128)(long long)(v[3] - b) << 48);
 }
+
+// comp_fixed (plain.hpp) of a component's columns: what does not depend on the
+// column (the biases and the rounding of the first shift, as one 128-bit
+// number) is made once, and the sums stay unsigned.  About half the
+// instructions of comp_fixed(join_limbs(..)) a column; the drains' instructions
+// are what the column kernel waits for (8192 unknowns (3-D) x 64: 327 -> 293 us).
+struct CompScale {
+    unsigned __int128 add;
+    unsigned long long kappa;
+    int shift;  // 1 .. 63
+    __device__ __forceinline__ CompScale(unsigned long long weights, int shift_, unsigned long long kappa_)
+        : kappa(kappa_), shift(shift_) {
+        const unsigned __int128 b = weights * kBias;
+        add = (unsigned __int128)(1ull << (shift - 1)) - (b + (b << 16) + (b << 32) + (b << 48));
+    }
+    __device__ __forceinline__ long long operator()(const unsigned long long (&v)[4]) const {
+        const unsigned __int128 r = add + v[0] + ((unsigned __int128)v[1] << 16) + ((unsigned __int128)v[2] << 32) +
+                                    ((unsigned __int128)v[3] << 48);
+        const uint32_t w0 = uint32_t(r), w1 = uint32_t(r >> 32), w2 = uint32_t(r >> 64), w3 = uint32_t(r >> 96);
+        const bool far = shift >= 32;  // (a funnel shift takes its low five bits)
+        const uint32_t lo = __funnelshift_r(far ? w1 : w0, far ? w2 : w1, uint32_t(shift));
+        const uint32_t hi = __funnelshift_r(far ? w2 : w1, far ? w3 : w2, uint32_t(shift));
+        const unsigned long long a = ((unsigned long long)hi << 32) | lo;
+        // signed a times unsigned kappa: the high 64 bits, rounded
+        const unsigned __int128 p = (unsigned __int128)a * kappa;
+        const unsigned long long q = (unsigned long long)(p >> 64) - (int(hi) < 0 ? kappa : 0ull);
+        return (long long)(q + ((unsigned long long)p >> 63));
+    }
+};
 
 // Half a tile row: 32 digits of one plane (shared address `src`, fragment
 // order: 32 bytes, or 16 for a nibble plane) as f16 operands d 2^-24 in the
@@ -611,17 +641,13 @@ __global__ void __launch_bounds__(kThreads, 1)
             const unsigned long long kappa = ((unsigned long long)rec.w << 32) | rec.z;
             long long* out = W.v + (long long)int(rec.x) * pv + c0;
             if (T.nparts == 1) {
+                const CompScale fixed(weights, max(shift, 1), kappa);
                 long long u[C::kPer];
 #pragma unroll
-                for (int r = 0; r < C::kPer; ++r) u[r] = comp_fixed(join_limbs(v[r], weights), shift, kappa);
-                if (lane < count) {
-                    if constexpr (C::kPer == 1) {
-                        out[0] = u[0];
-                    } else {
-#pragma unroll
-                        for (int r = 0; r < C::kPer; r += 2)
-                            *reinterpret_cast<longlong2*>(out + r) = make_longlong2(u[r], u[r + 1]);
-                    }
+                for (int r = 0; r < C::kPer; ++r) u[r] = fixed(v[r]);
+                if (lane < count && c0 < pv) {
+                    if constexpr (C::kPer == 1) out[0] = u[0];
+                    else *reinterpret_cast<longlong2*>(out) = make_longlong2(u[0], u[1]);
                 }
                 continue;
             }
@@ -1013,7 +1039,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 int comp, info;
                 asm volatile("ld.shared.v2.b32 {%0,%1}, [%2];" : "=r"(comp), "=r"(info) : "r"(rec_ring + uint32_t(((i & 3) * kS + k) * 1024)) : "memory");
                 const bool none = comp < 0 || slot0 + 32 * k >= q[3] >> 24;  // (-1: a slot past the k axis)
-                const long long* p = W.v + (long long)max(comp, 0) * pv + (q[3] & 0xFFFFFF) * R + pair * 2;
+                const long long* p = W.v + (long long)max(comp, 0) * pv + min((q[3] & 0xFFFFFF) * R + pair * 2, pv - 2);  // (past the last: not read)
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(v_ring + uint32_t(((i & 3) * kS + k) * 2048)), "l"(p)
                              : "memory");
                 sh[k] = (sh[k] & 0x00FFFFFFu) | uint32_t(none ? 63 : (info >> 8) & 63) << 24;
@@ -1088,45 +1114,52 @@ __global__ void __launch_bounds__(64) tc_combine_kernel(Arena A, Work W, double*
 }
 
 template <int R>
-cudaError_t launch(const TcArgs& a, cudaStream_t s, void (*mark)(void*, int), void* ctx) {
+cudaError_t launch_column(const TcArgs& a, cudaStream_t s) {
     const int groups = (a.rhs + R - 1) / R;
-    const long long cj = (long long)a.n_items * groups, rj = (long long)a.n_row_items * groups;
-    if (cj > INT32_MAX || rj > INT32_MAX) return cudaErrorInvalidValue;
-    cudaError_t e = cudaSuccess;
-    if (a.n_items > 0 || a.n_dense > 0)
-        e = launch_pdl(tc_column_kernel<R>, dim3(unsigned(a.sms)), dim3(kThreads), size_t(ColSmem<R>::kBytes), s, a.A, a.W,
-                       a.n_items, groups, a.n_dense, a.rhs, a.pv, a.n, a.n_pad, a.n_split, a.n_dslices, a.status);
-    if (mark) mark(ctx, 2);
-    if (e == cudaSuccess && rj > 0)
-        e = launch_pdl(tc_row_kernel<R>, dim3(unsigned(rj < a.sms ? rj : a.sms)), dim3(kThreads), size_t(RowSmem<R>::kBytes),
-                       s, a.A, a.W, a.n_row_items, groups, a.rhs, a.pv, a.n_parts, a.status);
-    if (e == cudaSuccess)
-        e = launch_pdl(tc_combine_kernel, dim3(unsigned(a.n_tiles), unsigned(a.rhs)), dim3(64), 0, s, a.A, a.W, a.y,
-                       a.n_parts, a.n_dslices, a.ld);
-    return e;
+    if ((long long)a.n_items * groups > INT32_MAX) return cudaErrorInvalidValue;
+    if (a.n_items == 0 && a.n_dense == 0) return cudaSuccess;
+    return launch_pdl(tc_column_kernel<R>, dim3(unsigned(a.sms)), dim3(kThreads), size_t(ColSmem<R>::kBytes), s, a.A, a.W,
+                      a.n_items, groups, a.n_dense, a.rhs, a.pv, a.n, a.n_pad, a.n_split, a.n_dslices, a.status);
+}
+template <int R>
+cudaError_t launch_row(const TcArgs& a, cudaStream_t s) {
+    const int groups = (a.rhs + R - 1) / R;
+    const long long jobs = (long long)a.n_row_items * groups;
+    if (jobs > INT32_MAX) return cudaErrorInvalidValue;
+    if (jobs == 0) return cudaSuccess;
+    return launch_pdl(tc_row_kernel<R>, dim3(unsigned(jobs < a.sms ? jobs : a.sms)), dim3(kThreads),
+                      size_t(RowSmem<R>::kBytes), s, a.A, a.W, a.n_row_items, groups, a.rhs, a.pv, a.n_parts, a.status);
 }
 
-template <int R>
-cudaError_t allow_smem() {
-    cudaError_t e = cudaFuncSetAttribute(tc_column_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, ColSmem<R>::kBytes);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(tc_row_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, RowSmem<R>::kBytes);
-    return e;
+template <class K>
+cudaError_t allow_smem(K* kernel, int bytes) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
 }  // namespace
 }  // namespace tc
 
-int tc_columns(int rhs) { return rhs > 4 ? 8 : 4; }
-
 cudaError_t tc_setup() {
-    cudaError_t e = tc::allow_smem<4>();
-    if (e == cudaSuccess) e = tc::allow_smem<8>();
+    using namespace tc;
+    cudaError_t e = allow_smem(tc_column_kernel<4>, ColSmem<4>::kBytes);
+    if (e == cudaSuccess) e = allow_smem(tc_column_kernel<8>, ColSmem<8>::kBytes);
+    if (e == cudaSuccess) e = allow_smem(tc_row_kernel<4>, RowSmem<4>::kBytes);
+    if (e == cudaSuccess) e = allow_smem(tc_row_kernel<8>, RowSmem<8>::kBytes);
     return e;
 }
 
 cudaError_t tc_launch(const TcArgs& a, cudaStream_t s, void (*mark)(void*, int), void* ctx) {
-    return tc_columns(a.rhs) == 4 ? tc::launch<4>(a, s, mark, ctx) : tc::launch<8>(a, s, mark, ctx);
+    using namespace tc;
+    // four columns at once cost less than eight (8192 unknowns (3-D): 82 us for 3
+    // or 4 columns, 92 for 5 .. 8)
+    const bool few = a.rhs <= 4;
+    cudaError_t e = few ? launch_column<4>(a, s) : launch_column<8>(a, s);
+    if (mark) mark(ctx, 2);
+    if (e == cudaSuccess) e = few ? launch_row<4>(a, s) : launch_row<8>(a, s);
+    if (e == cudaSuccess)
+        e = launch_pdl(tc_combine_kernel, dim3(unsigned(a.n_tiles), unsigned(a.rhs)), dim3(64), 0, s, a.A, a.W, a.y,
+                       a.n_parts, a.n_dslices, a.ld);
+    return e;
 }
 
 }  // namespace qhg

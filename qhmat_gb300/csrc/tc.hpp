@@ -15,9 +15,6 @@ struct TcArgs {
     int* status;
 };
 
-// Right-hand-side columns the kernels take at once for an apply of rhs
-// columns (rows of V hold a multiple of it).
-int tc_columns(int rhs);
 // Once per device: the kernels' shared memory.
 cudaError_t tc_setup();
 // Column, row and combine kernels in stream order; mark(ctx, 2), if given, is
