@@ -1543,27 +1543,23 @@ int check_rhs(const qh_matrix* m, size_t rhs) {
 namespace {
 
 // Makes the pages of a host buffer that is about to be written as a whole
-// present, on four threads (one write per page; the operating system clears the
-// page: a new 33 MB buffer took 1.1 ms on one thread, 0.41 ms on four, 0.53 ms
-// on eight, and 1.9 ms within a device-to-host copy).
+// present, on up to four threads, the caller's among them (one write per page;
+// the operating system clears the page: a new 33 MB buffer took 1.1 ms on one
+// thread, 0.41 ms on four, 0.53 ms on eight, and 1.9 ms within a
+// device-to-host copy).  Below 4 MB the copy does it as fast.
 class PagePopulator {
 public:
     PagePopulator(void* p, size_t bytes) {
         if (!p || bytes < kPart) return;
-        const size_t n = std::min<size_t>({bytes / kPart, kThreads, std::max(1u, std::thread::hardware_concurrency())});
-        const size_t page = sysconf(_SC_PAGESIZE) > 0 ? size_t(sysconf(_SC_PAGESIZE)) : 4096;
+        const size_t n = std::max<size_t>(1, std::min<size_t>({bytes / kPart, kThreads, std::thread::hardware_concurrency()}));
         auto* b = static_cast<uint8_t*>(p);
-        for (size_t k = 0; k < n; ++k)
+        for (size_t k = 0; k + 1 < n; ++k)
             try {
-                threads_[k] = std::thread([b, bytes, page, k, n] {
-                    const size_t at = bytes / n * k, end = k + 1 == n ? bytes : bytes / n * (k + 1);
-                    for (size_t i = at; i < end; i += page) *static_cast<volatile uint8_t*>(b + i) = 0;
-                    b[end - 1] = 0;  // (the buffer need not start on a page: a single absent
-                                     // page costs the copy 0.7 ms)
-                });
+                threads_[k] = std::thread([=] { touch(b + bytes / n * k, bytes / n); });
             } catch (const std::system_error&) {
-                return;  // no more threads: the copy populates the rest
+                break;  // no more threads: the copy populates that part
             }
+        touch(b + bytes / n * (n - 1), bytes - bytes / n * (n - 1));
     }
     ~PagePopulator() { wait(); }
     void wait() {
@@ -1573,7 +1569,13 @@ public:
 
 private:
     static constexpr size_t kThreads = 4, kPart = size_t(4) << 20;  // at least kPart bytes for a thread
-    std::thread threads_[kThreads];
+    static void touch(uint8_t* p, size_t bytes) {
+        const size_t page = sysconf(_SC_PAGESIZE) > 0 ? size_t(sysconf(_SC_PAGESIZE)) : 4096;
+        for (size_t i = 0; i < bytes; i += page) *static_cast<volatile uint8_t*>(p + i) = 0;
+        // (the buffer need not start on a page: a single absent page costs the copy 0.7 ms)
+        *static_cast<volatile uint8_t*>(p + bytes - 1) = 0;
+    }
+    std::thread threads_[kThreads - 1];
 };
 
 }  // namespace
@@ -1937,24 +1939,28 @@ int qh_matrix_reconstruct(const qh_matrix* m, double* out, size_t out_count, int
             }
         }
         if (tiles > INT32_MAX) return fail(QH_EOVERFLOW, "CUDA launch grid too large");
-        // one allocation: factors, bases, blocks, and the output if on the host
-        size_t bytes = 0;
-        auto take = [&](size_t b) {
-            const size_t o = bytes;
-            bytes += align256(std::max<size_t>(b, 1));
-            return o;
-        };
-        const size_t o_left = take(8 * size_t(ltotal)), o_right = take(8 * size_t(rtotal));
-        const size_t o_lb = take(8 * size_t(m->L.n_comp)), o_rb = take(8 * size_t(m->L.n_comp));
-        const size_t o_blocks = take(sizeof(DenseOut) * size_t(nb)), o_out = take(out_on_device ? 0 : 8 * n * n);
-        uint8_t* buf = nullptr;
-        if (cudaMalloc(&buf, bytes) != cudaSuccess) return fail(QH_ERUNTIME, "cudaMalloc: out of device memory");
-        auto* left = reinterpret_cast<double*>(buf + o_left);
-        auto* right = reinterpret_cast<double*>(buf + o_right);
-        auto* lb = reinterpret_cast<long long*>(buf + o_lb);
-        auto* rb = reinterpret_cast<long long*>(buf + o_rb);
-        auto* d_blocks = reinterpret_cast<DenseOut*>(buf + o_blocks);
-        double* d_out = out_on_device ? out : reinterpret_cast<double*>(buf + o_out);
+        // one allocation (separate ones were slower at every order): factors,
+        // bases, blocks, and the output if on the host
+        const size_t parts[5] = {8 * size_t(ltotal), 8 * size_t(rtotal), 16 * size_t(m->L.n_comp),
+                                 sizeof(DenseOut) * size_t(nb), out_on_device ? 0 : 8 * n * n};
+        size_t at[5], bytes = 0;
+        for (int i = 0; i < 5; ++i) {
+            at[i] = bytes;
+            bytes += align256(std::max<size_t>(parts[i], 1));
+        }
+        struct Scratch {
+            uint8_t* p = nullptr;
+            ~Scratch() {
+                if (p) cudaFree(p);
+            }
+        } buf;
+        if (cudaMalloc(&buf.p, bytes) != cudaSuccess) return fail(QH_ERUNTIME, "cudaMalloc: out of device memory");
+        auto* left = reinterpret_cast<double*>(buf.p + at[0]);
+        auto* right = reinterpret_cast<double*>(buf.p + at[1]);
+        auto* lb = reinterpret_cast<long long*>(buf.p + at[2]);
+        auto* rb = lb + m->L.n_comp;
+        auto* d_blocks = reinterpret_cast<DenseOut*>(buf.p + at[3]);
+        double* d_out = out_on_device ? out : reinterpret_cast<double*>(buf.p + at[4]);
         cudaError_t e = cudaMemcpy(d_blocks, blocks.data(), sizeof(DenseOut) * blocks.size(), cudaMemcpyHostToDevice);
         if (e == cudaSuccess && n_lr) {
             factor_base_kernel<<<unsigned(n_lr), 32>>>(m->A, n_lr, d_blocks, lb, rb);
@@ -1969,9 +1975,7 @@ int qh_matrix_reconstruct(const qh_matrix* m, double* out, size_t out_count, int
         PagePopulator(out_on_device ? nullptr : out, 8 * n * n).wait();
         if (e == cudaSuccess)
             e = out_on_device ? cudaDeviceSynchronize() : cudaMemcpy(out, d_out, 8 * n * n, cudaMemcpyDeviceToHost);
-        const int rc = e == cudaSuccess ? QH_OK : cuda_fail(e, "reconstruct");
-        cudaFree(buf);
-        return rc;
+        return e == cudaSuccess ? QH_OK : cuda_fail(e, "reconstruct");
     });
 }
 
