@@ -180,6 +180,48 @@ __global__ void __launch_bounds__(256) prep_limbs_kernel(Arena A, Work W, const 
     limbs_block(W, n, n_pad, gridDim.x, blockIdx.y, blockIdx.x, gridDim.x, s_m);
 }
 
+// prep_x and x_limbs for an order of at most kPrepCluster * kPrepThreads: a
+// cluster of blocks per column, a thread per clustered entry, which keeps it
+// in a register until the column's exponent is known (block maxima exchanged
+// through distributed shared memory).  Bound by latency: no grid-wide
+// synchronisation, no second read, and it is launched while its predecessor
+// ends, which a cooperative launch is not.
+constexpr int kPrepCluster = 8, kPrepThreads = 1024;
+__global__ void __cluster_dims__(kPrepCluster, 1, 1) __launch_bounds__(kPrepThreads)
+    prep_cluster_kernel(Arena A, Work W, const double* __restrict__ x, int n, long long ld, int* zero, int n_zero,
+                        int* status, int n_pad) {
+    __shared__ int s_m[kPrepThreads / 32], s_all[kPrepCluster];
+    auto cluster = cooperative_groups::this_cluster();
+    cluster.barrier_arrive();
+    pdl_trigger();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, p = blockIdx.y;
+    const int k = int(blockIdx.x) * kPrepThreads + int(threadIdx.x);
+    const int src = k < n ? __ldg(A.perm + k) : -1;
+    pdl_wait();
+    double v = src >= 0 ? x[(long long)src * ld + p] : 0.0;  // (plain load)
+    constexpr int kStep = kPrepCluster * kPrepThreads;
+    for (long long i = (long long)p * kStep + k; i < n_zero; i += (long long)gridDim.y * kStep) zero[i] = 0;
+    const int e = exp_field(v);
+    if (e == 0x7FF) v = 0.0;
+    if (__any_sync(0xFFFFFFFFu, e == 0x7FF) && lane == 0 && status) atomicOr(status, kStatusNonfinite);
+    int m = __reduce_max_sync(0xFFFFFFFFu, e == 0x7FF ? 0 : e);
+    if (lane == 0) s_m[warp] = m;
+    __syncthreads();
+    cluster.barrier_wait();  // every block runs
+    if (warp == 0) {
+        m = __reduce_max_sync(0xFFFFFFFFu, s_m[lane]);
+        if (lane < kPrepCluster) *cluster.map_shared_rank(&s_all[blockIdx.x], unsigned(lane)) = m;
+    }
+    cluster.sync();
+    int xe = 0;
+#pragma unroll
+    for (int i = 0; i < kPrepCluster; ++i) xe = max(xe, s_all[i]);
+    if (k == 0) W.xe[p] = xe;
+    if (k < n) W.xc[(long long)p * n + k] = v;
+    if (k < n_pad) W.xq[(long long)p * n_pad + k] = to_limbs(xe ? to_fixed(v, xe) : 0);
+}
+static_assert(kPrepThreads == 32 * 32, "one warp reduces the warps' maxima");
+
 // Bring a line into L1 ahead of its use (no register waits on it).
 __device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
@@ -1465,7 +1507,15 @@ int launch_chunk(const qh_matrix* m, const double* x, double* y, size_t rhs, lon
     int* zero = reinterpret_cast<int*>(w + P.zero0);
     const int n_zero = int(P.zero_bytes / 4);
     cudaError_t e;
-    if (static_cast<long long>(P.nblk) * irhs <= m->prep_coop_max) {
+    // One cluster per column where its threads reach and all clusters fit at once
+    // (two blocks per SM).  Whole applies, us, cooperative / cluster: 2048 x 1
+    // 18.5 / 16.2, 2048 x 4 26.9 / 25.1, 8000 x 1 32.8 / 30.6, 8000 x 16 90.5 / 87.6;
+    // two entries a thread, 12345 x 1 40.8 / 40.9; more clusters than fit,
+    // 8000 x 64 309 / 313.
+    if (n_pad <= kPrepCluster * kPrepThreads && kPrepCluster * irhs <= 2 * m->sms) {
+        e = launch_pdl(prep_cluster_kernel, dim3(kPrepCluster, unsigned(rhs)), dim3(kPrepThreads), 0, s, m->A, W, x, n, ld,
+                       zero, n_zero, status, n_pad);
+    } else if (static_cast<long long>(P.nblk) * irhs <= m->prep_coop_max) {
         // one cooperative launch: prep, a grid-wide synchronisation, limbs
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(unsigned(P.nblk), unsigned(rhs));

@@ -13,8 +13,7 @@
 //                        2-D tensor copies (cp.async.bulk.tensor, 128-byte
 //                        swizzle) straight into the B operand layout;
 //   pf_column_kernel     T = Q^T X' for 128 components sharing a column range;
-//                        u = (s^P s^Q) T in FP64 (the per-component scale),
-//                        stored as FP32 per row-side slot;
+//                        u = (s^P s^Q) T in FP32, stored per row-side slot;
 //   pf_row_kernel        y = P U' per 128-row tile (U' = three f16 limbs of u
 //                        on a per-column exponent), plus the dense diagonal
 //                        blocks as three f16 limb tiles against X' limbs;
@@ -23,10 +22,10 @@
 //                        order (deterministic), scattered through perm.
 //
 // Both streaming kernels are persistent and warp-specialised: one warp issues
-// the bulk and tensor copies into a ring of shared-memory stages, six (column)
-// or eight (row) warps
-// turn digit bytes (and U) into f16 operand tiles, one thread issues the
-// MMAs, four warps drain the accumulators from tensor memory.  Every wait is
+// the bulk and tensor copies into a ring of shared-memory stages, eight warps
+// turn digit bytes into f16 operand tiles (in the row kernel, four more turn U
+// into B tiles), one thread issues the
+// MMAs, eight warps drain the accumulators from tensor memory.  Every wait is
 // bounded; a wait that gives up sets QH_STATUS_TIMEOUT and the block winds
 // down (after a bounded drain of its copies and MMAs) instead of hanging.
 //
