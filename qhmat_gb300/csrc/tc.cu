@@ -266,7 +266,7 @@ __device__ __forceinline__ __int128 join_limbs(const unsigned long long (&v)[4],
 // column (the biases and the rounding of the first shift, as one 128-bit
 // number) is made once, and the sums stay unsigned.  About half the
 // instructions of comp_fixed(join_limbs(..)) a column; the drains' instructions
-// are what the column kernel waits for (8192 unknowns (3-D) x 64: 327 -> 293 us).
+// are what the column kernel waits for (8192 unknowns (3-D) x 64: 327 -> 318 us).
 struct CompScale {
     unsigned __int128 add;
     unsigned long long kappa;
@@ -621,7 +621,11 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const uint32_t word = *reinterpret_cast<volatile uint32_t*>(&S.segment[buf]);
                 end = (word >> 8) & 1u;
                 const int P = int(word & 15u);
-                const uint32_t base = tmem + (uint32_t(32 * sub) << 16) + uint32_t(buf * kAccStride + e * 8 * C::kPer);
+                // (always the set's columns: no item has more planes than a set holds.
+                // Without the test ptxas keeps both sets' addresses and spills sums:
+                // 8192 unknowns (3-D) x 64, column kernel 318 us instead of 293)
+                const int set = P <= kAccStride / C::N ? buf * kAccStride : 0;
+                const uint32_t base = tmem + (uint32_t(32 * sub) << 16) + uint32_t(set + e * 8 * C::kPer);
                 if (count > 0)
 #pragma unroll 1
                     for (int m = 0; m < P; ++m) {
