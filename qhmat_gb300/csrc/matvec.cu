@@ -1973,6 +1973,7 @@ int qh_matrix_reconstruct(const qh_matrix* m, double* out, size_t out_count, int
         // blocks' tiles and factors (component-major)
         std::vector<DenseOut> blocks(static_cast<size_t>(nb));
         long long tiles = 0, ltotal = 0, rtotal = 0;
+        size_t area = 0;  // entries inside the blocks, which do not overlap
         auto tiles_of = [](long long rows, long long cols) {
             return ((rows + kDenseTile - 1) / kDenseTile) * ((cols + kDenseTile - 1) / kDenseTile);
         };
@@ -1983,9 +1984,11 @@ int qh_matrix_reconstruct(const qh_matrix* m, double* out, size_t out_count, int
                 ltotal += (long long)d.rank * d.m;
                 rtotal += (long long)d.rank * d.n;
                 tiles += tiles_of(d.m, d.n);
+                area += size_t(d.m) * size_t(d.n);
             } else {
                 const DenseDesc& d = m->dd[size_t(b - n_lr)];
                 tiles += tiles_of(d.m, d.n);
+                area += size_t(d.m) * size_t(d.n);
             }
         }
         if (tiles > INT32_MAX) return fail(QH_EOVERFLOW, "CUDA launch grid too large");
@@ -2012,6 +2015,9 @@ int qh_matrix_reconstruct(const qh_matrix* m, double* out, size_t out_count, int
         auto* d_blocks = reinterpret_cast<DenseOut*>(buf.p + at[3]);
         double* d_out = out_on_device ? out : reinterpret_cast<double*>(buf.p + at[4]);
         cudaError_t e = cudaMemcpy(d_blocks, blocks.data(), sizeof(DenseOut) * blocks.size(), cudaMemcpyHostToDevice);
+        // the blocks of one matrix cover it; those of a block-diagonal handle
+        // (qh_matrix_from_batch) do not, and what lies outside them is zero
+        if (e == cudaSuccess && area < n * n) e = cudaMemsetAsync(d_out, 0, 8 * n * n, nullptr);
         if (e == cudaSuccess && n_lr) {
             factor_base_kernel<<<unsigned(n_lr), 32>>>(m->A, n_lr, d_blocks, lb, rb);
             e = launch_decode<double>(m->A, m->L.n_tasks, rb, right, m->L.n_units, lb, left);
