@@ -1042,11 +1042,15 @@ __global__ void __launch_bounds__(kThreads, 1)
             for (int k = 0; k < kS; ++k) {
                 int comp, info;
                 asm volatile("ld.shared.v2.b32 {%0,%1}, [%2];" : "=r"(comp), "=r"(info) : "r"(rec_ring + uint32_t(((i & 3) * kS + k) * 1024)) : "memory");
-                const bool none = comp < 0 || slot0 + 32 * k >= q[3] >> 24;  // (-1: a slot past the k axis)
+                // a slot past the k axis (-1) has U = 0: no bytes of V are read
+                // for it, the copy writes zeros (its digits are not zero, and V
+                // of a component that no block holds is never written)
+                const bool none = comp < 0 || slot0 + 32 * k >= q[3] >> 24;
                 const long long* p = W.v + (long long)max(comp, 0) * pv + min((q[3] & 0xFFFFFF) * R + pair * 2, pv - 2);  // (past the last: not read)
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(v_ring + uint32_t(((i & 3) * kS + k) * 2048)), "l"(p)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(v_ring + uint32_t(((i & 3) * kS + k) * 2048)), "l"(p),
+                             "r"(none ? 0 : 16)
                              : "memory");
-                sh[k] = (sh[k] & 0x00FFFFFFu) | uint32_t(none ? 63 : (info >> 8) & 63) << 24;
+                sh[k] = (sh[k] & 0x00FFFFFFu) | uint32_t((info >> 8) & 63) << 24;
             }
         };
         pdl_wait();  // V of this apply
