@@ -38,6 +38,8 @@
 // split, so y is the same bit for bit whatever the number of columns.
 #include "tc.hpp"
 
+#include <algorithm>
+
 #include "tcgen05.hpp"
 
 namespace qhg {
@@ -1126,7 +1128,13 @@ cudaError_t launch_column(const TcArgs& a, cudaStream_t s) {
     const int groups = (a.rhs + R - 1) / R;
     if ((long long)a.n_items * groups > INT32_MAX) return cudaErrorInvalidValue;
     if (a.n_items == 0 && a.n_dense == 0) return cudaSuccess;
-    return launch_pdl(tc_column_kernel<R>, dim3(unsigned(a.sms)), dim3(kThreads), size_t(ColSmem<R>::kBytes), s, a.A, a.W,
+    // No more blocks than there is work for: an item and a column block each, or
+    // one dense part for each of a block's four dense warps.  A block holds a
+    // whole SM, which another stream's kernels could use (six matrices of 300
+    // unknowns, 3 columns, a stream each: 28.2 us an apply of all on a grid of every
+    // SM, 16.6 on this one, 24.6 on the column-by-column kernels).
+    const long long jobs = std::max((long long)a.n_items * groups, ((long long)a.n_dense * (a.rhs + 1) + 3) / 4);
+    return launch_pdl(tc_column_kernel<R>, dim3(unsigned(std::min<long long>(jobs, a.sms))), dim3(kThreads), size_t(ColSmem<R>::kBytes), s, a.A, a.W,
                       a.n_items, groups, a.n_dense, a.rhs, a.pv, a.n, a.n_pad, a.n_split, a.n_dslices, a.status);
 }
 template <int R>
