@@ -13,8 +13,10 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <limits>
 #include <numeric>
+#include <queue>
 #include <utility>
 
 namespace qhg {
@@ -887,6 +889,98 @@ Layout build_layout(const HostMatrix& m) {
     put(S.tc_steps, tc_steps);
     if (!tdense.empty()) std::memcpy(A.data() + S.tdense, tdense.data(), sizeof(TileDense) * tdense.size());
     return L;
+}
+
+std::vector<double> column_costs(const Layout& L) {
+    const auto* tasks = reinterpret_cast<const ColTask*>(L.arena.data() + L.sec.tasks);
+    std::vector<double> c(static_cast<size_t>(L.n_tasks));
+    for (size_t i = 0; i < c.size(); ++i) {
+        // (least squares over clock64 timings of every unit of a 32768-point
+        // kernel matrix, R^2 0.97): per unit (descriptor loads, the
+        // finalize), per pipeline step (copy latency not hidden by two
+        // stages), per chunk and per code byte; per 32 B rows written
+        // (timed alone), charged to every part of a split task since any
+        // of them may be the one that finishes it
+        const ColTask& T = tasks[i];
+        if (T.width == 0) {
+            c[i] = 1000.0 * double(T.n);  // dense unit: FP64, ~16k cycles for 16 columns
+            continue;
+        }
+        const double steps = double((T.nchunks + T.cps - 1) / T.cps);
+        c[i] = 4100.0 + 1415.0 * steps + 490.0 * T.nchunks + 0.194 * double(T.nchunks) * T.stride +
+               700.0 * double((T.ndest + 31) / 32) + (T.nparts > 1 ? 584.0 : 0.0);
+    }
+    return c;
+}
+
+std::vector<double> row_costs(const Layout& L) {
+    const auto* units = reinterpret_cast<const RowUnit*>(L.arena.data() + L.sec.units);
+    const uint8_t* info = L.arena.data() + L.sec.kp_info;
+    std::vector<double> c(static_cast<size_t>(L.n_units));
+    for (size_t i = 0; i < c.size(); ++i) {
+        // (clock64 timings of every unit of a 32768-point kernel matrix): per
+        // k-pair and per digit plane of it (MMAs, digit conversion), per
+        // pipeline step, per unit (descriptor, the 128-bit epilogue)
+        const RowUnit& U = units[i];
+        double planes = 0;
+        for (int k = 0; k < U.nkps; ++k) planes += info[U.kp_off + U.h + int64_t(k) * U.H] & 7;
+        c[i] = 2000.0 + 350.0 * U.nkps + 380.0 * planes + 300.0 * U.nsteps;
+    }
+    return c;
+}
+
+Schedule schedule_units(const std::vector<double>& costs, int warps) {
+    Schedule s;
+    std::vector<int32_t> idx(costs.size(), 0);
+    std::iota(idx.begin(), idx.end(), 0);
+    std::stable_sort(idx.begin(), idx.end(), [&](int32_t a, int32_t b) { return costs[size_t(a)] > costs[size_t(b)]; });
+    using Load = std::pair<double, int32_t>;
+    std::priority_queue<Load, std::vector<Load>, std::greater<Load>> heap;
+    for (int32_t w = 0; w < warps; ++w) heap.push({0.0, w});
+    std::vector<std::vector<int32_t>> lists(static_cast<size_t>(warps));
+    for (int32_t i : idx) {
+        Load l = heap.top();
+        heap.pop();
+        lists[size_t(l.second)].push_back(i);
+        l.first += costs[size_t(i)];
+        s.total += costs[size_t(i)];
+        s.longest = std::max(s.longest, l.first);
+        heap.push(l);
+    }
+    s.off.assign(size_t(warps) + 1, 0);
+    for (int32_t w = 0; w < warps; ++w) {
+        s.off[size_t(w)] = int32_t(s.order.size());
+        s.order.insert(s.order.end(), lists[size_t(w)].begin(), lists[size_t(w)].end());
+    }
+    s.off[size_t(warps)] = int32_t(s.order.size());
+    return s;
+}
+
+KernelChoice kernel_choice(const Layout& L, const Schedule& columns, const Schedule& rows, int sms) {
+    KernelChoice c;
+    // column by column: the warps' mean load, and what the longest has beyond it
+    // (cycles at 2.07 GHz); x and y; B rows written and read
+    const double mean = (columns.total + rows.total) / (16.0 * sms) / 2070.0;
+    const double longest = (columns.longest + rows.longest) / 2070.0;
+    c.column = 0.69 * mean + 0.44 * (longest - mean) + 1.7e-4 * double(L.order) + 8.6e-6 * double(L.n_slots);
+    const auto* items = reinterpret_cast<const TcItem*>(L.arena.data() + L.sec.tc_items);
+    const auto* row_items = reinterpret_cast<const TcRowItem*>(L.arena.data() + L.sec.tc_row_items);
+    // (a step holds two chunks of at most two planes, or one of more)
+    for (int32_t i = 0; i < L.n_tc_items; ++i)
+        c.steps += (items[i].info & 255) <= 2 ? (items[i].nchunks + 1) / 2 : items[i].nchunks;
+    for (int32_t i = 0; i < L.n_tc_row_items; ++i) c.row_steps += row_items[i].nsteps;
+    c.steps /= sms, c.row_steps /= sms;
+    c.items = double(L.n_tc_items) / sms, c.dense = double(L.n_dense_units) / sms;
+    return c;
+}
+
+bool KernelChoice::tensor(size_t rhs) const {
+    if (rhs < 3) return false;
+    const double p = double(rhs), groups = double((rhs + 7) / 8);
+    const double several =
+        rhs <= 4 ? 15.6 + 0.47 * steps + 0.44 * items + 0.82 * row_steps + 0.43 * p * dense
+                 : 16.3 + groups * (0.22 * steps + 1.05 * items + 0.74 * row_steps) + 0.06 * steps + 0.61 * p * dense;
+    return several < 14.0 + p * column;
 }
 
 }  // namespace qhg

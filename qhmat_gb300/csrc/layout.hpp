@@ -292,6 +292,44 @@ struct Layout {
 
 Layout build_layout(const HostMatrix& m);
 
+// SM cycles of each column task / row unit of the column-by-column kernels with
+// every warp of the device resident (16 an SM).
+std::vector<double> column_costs(const Layout& L);
+std::vector<double> row_costs(const Layout& L);
+
+// Longest-first assignment of units to warps: each goes to the warp with the
+// least work so far.  The permutation is warp-major (each warp's units heaviest
+// first), with the warps' `warps + 1` offsets.
+struct Schedule {
+    std::vector<int32_t> order, off;
+    double total = 0, longest = 0;  // cycles: of all units, of the warp with the most
+};
+Schedule schedule_units(const std::vector<double>& costs, int warps);
+
+// Which kernels an apply of `rhs` columns takes: the column-by-column ones
+// (matvec.cu), which stream and convert every code once per column, or the
+// tensor-memory ones (tc.cu), which do it once per four (up to four columns) or
+// eight columns, in items of 128 rows and steps with a fixed handshake cost.
+// Both give the same bits.  Where the line lies depends on how full the items
+// are, so the times of both are predicted, in us, from the work lists; the
+// coefficients are least-squares fits to whole applies of 40 matrices (1-D, 2-D
+// and 3-D, 300 .. 100000 unknowns, leaves of 16 .. 128) with 3 .. 33 columns, 8 %
+// and 5 % off in the mean.  Column by column / tensor memory, us:
+//                          3 columns   4           5           8           9           16
+//   2048 (1-D, leaf 32)    32 / 25     40 / 25     48 / 28     71 / 28     81 / 35     139 / 35
+//   16384 (1-D, leaf 16)   87 / 134    113 / 137   137 / 161   212 / 169   236 / 300   412 / 321
+//   100000 (1-D, leaf 64)  303 / 489   394 / 495   486 / 548   765 / 582   862 / 1037  1525 / 1131
+//   9001 (2-D, leaf 32)    108 / 108   140 / 110   171 / 125   266 / 132   303 / 220   520 / 232
+//   16384 (2-D, leaf 64)   112 / 87    146 / 87    183 / 98    280 / 106   316 / 164   551 / 185
+//   8192 (3-D, leaf 64)    133 / 82    174 / 82    212 / 91    332 / 92    372 / 158   644 / 163
+// One and two columns never take them (32768 (2-D) x 1: 81 / 155, 9001 x 2: 77 / 105).
+struct KernelChoice {
+    double column = 0;                                      // us a column
+    double steps = 0, items = 0, row_steps = 0, dense = 0;  // per SM, of one pass over the codes
+    bool tensor(size_t rhs) const;
+};
+KernelChoice kernel_choice(const Layout& L, const Schedule& columns, const Schedule& rows, int sms);
+
 // Words of the bit string of `rows` codes of width w.
 inline uint64_t words_for_bits(uint64_t rows, int w) { return (rows * uint64_t(w) + 31) / 32; }
 

@@ -29,8 +29,9 @@
 //   combine_kernel     thread per row: dense row sums in column order plus
 //                      the partials -> y (one conversion).
 //
-// Applies of three columns and more take the column, row and combine kernels of
-// tc.cu instead (the same integers on the 5th-generation tensor cores).
+// Most applies of three columns and more take the column, row and combine
+// kernels of tc.cu instead (the same integers on the 5th-generation tensor
+// cores; KernelChoice in layout.hpp).
 //
 // The only rounding steps are the fixed-point conversions of x and u (2^-63
 // of the column's largest |x|, ~2^-62 of the component's and of the tile's
@@ -47,8 +48,6 @@
 #include <cstring>
 #include <mutex>
 #include <new>
-#include <numeric>
-#include <queue>
 #include <type_traits>
 #include <string>
 #include <system_error>
@@ -1171,6 +1170,7 @@ struct qh_matrix {
     // warp_off[w] .. warp_off[w + 1] of the (reordered) task (unit) array
     int* sched = nullptr;
     int col_grid = 0, row_grid = 0;
+    KernelChoice choice;
     StatusWords words;  // of qh_matmul_device_checked
     std::vector<LowRankDesc> lr;  // host copies of the blocks (reconstruct)
     std::vector<DenseDesc> dd;
@@ -1229,36 +1229,6 @@ int check_device(int device) {
     return QH_OK;
 }
 
-// Longest-first assignment of n units (cost(i)) to W warps: each unit goes to
-// the warp with the least work so far.  Returns the permutation (warp-major,
-// each warp's units heaviest first) and the W + 1 warp offsets.
-template <class F>
-void schedule(int n, int W, F cost, std::vector<int32_t>& order, std::vector<int32_t>& off) {
-    std::vector<int32_t> idx(static_cast<size_t>(n), 0);
-    std::iota(idx.begin(), idx.end(), 0);
-    std::vector<double> c(static_cast<size_t>(n), 0.0);
-    for (int i = 0; i < n; ++i) c[size_t(i)] = cost(i);
-    std::stable_sort(idx.begin(), idx.end(), [&](int32_t a, int32_t b) { return c[size_t(a)] > c[size_t(b)]; });
-    using Load = std::pair<double, int32_t>;
-    std::priority_queue<Load, std::vector<Load>, std::greater<Load>> heap;
-    for (int32_t w = 0; w < W; ++w) heap.push({0.0, w});
-    std::vector<std::vector<int32_t>> lists(static_cast<size_t>(W));
-    for (int32_t i : idx) {
-        Load l = heap.top();
-        heap.pop();
-        lists[size_t(l.second)].push_back(i);
-        l.first += c[size_t(i)];
-        heap.push(l);
-    }
-    order.clear();
-    off.assign(size_t(W) + 1, 0);
-    for (int32_t w = 0; w < W; ++w) {
-        off[size_t(w)] = int32_t(order.size());
-        order.insert(order.end(), lists[size_t(w)].begin(), lists[size_t(w)].end());
-    }
-    off[size_t(W)] = int32_t(order.size());
-}
-
 template <class T>
 void permute(T* a, const std::vector<int32_t>& order) {
     std::vector<T> tmp(a, a + order.size());
@@ -1293,36 +1263,13 @@ int upload(Layout&& L, int device, qh_matrix** out) {
         m->row_grid = std::max(1, std::min((Lm.n_units + kWarps - 1) / kWarps, m->sms * 2));
         auto* tasks = reinterpret_cast<ColTask*>(Lm.arena.data() + Lm.sec.tasks);
         auto* units = reinterpret_cast<RowUnit*>(Lm.arena.data() + Lm.sec.units);
-        const uint8_t* kpi = Lm.arena.data() + Lm.sec.kp_info;
-        std::vector<int32_t> corder, coff, rorder, roff;
-        schedule(Lm.n_tasks, m->col_grid * kWarps, [&](int i) {
-            // SM cycles of a column unit with all warps resident (least
-            // squares over clock64 timings of every unit of a 32768-point
-            // kernel matrix, R^2 0.97): per unit (descriptor loads, the
-            // finalize), per pipeline step (copy latency not hidden by two
-            // stages), per chunk and per code byte; per 32 B rows written
-            // (timed alone), charged to every part of a split task since any
-            // of them may be the one that finishes it
-            const ColTask& T = tasks[i];
-            if (T.width == 0) return 1000.0 * double(T.n);  // dense unit: FP64, ~16k cycles for 16 columns
-            const double steps = double((T.nchunks + T.cps - 1) / T.cps);
-            return 4100.0 + 1415.0 * steps + 490.0 * T.nchunks + 0.194 * double(T.nchunks) * T.stride +
-                   700.0 * double((T.ndest + 31) / 32) + (T.nparts > 1 ? 584.0 : 0.0);
-        }, corder, coff);
-        schedule(Lm.n_units, m->row_grid * kWarps, [&](int i) {
-            // SM cycles of a row unit with all warps resident (clock64
-            // timings of every unit of a 32768-point kernel matrix): per
-            // k-pair and per digit plane of it (MMAs, digit conversion), per
-            // pipeline step, per unit (descriptor, the 128-bit epilogue)
-            const RowUnit& U = units[i];
-            double planes = 0;
-            for (int k = 0; k < U.nkps; ++k) planes += kpi[U.kp_off + U.h + int64_t(k) * U.H] & 7;
-            return 2000.0 + 350.0 * U.nkps + 380.0 * planes + 300.0 * U.nsteps;
-        }, rorder, roff);
-        permute(tasks, corder);
-        permute(units, rorder);
-        std::vector<int32_t> sched(coff);
-        sched.insert(sched.end(), roff.begin(), roff.end());
+        const Schedule col = schedule_units(column_costs(Lm), m->col_grid * kWarps);
+        const Schedule row = schedule_units(row_costs(Lm), m->row_grid * kWarps);
+        permute(tasks, col.order);
+        permute(units, row.order);
+        m->choice = kernel_choice(Lm, col, row, m->sms);
+        std::vector<int32_t> sched(col.off);
+        sched.insert(sched.end(), row.off.begin(), row.off.end());
         cudaError_t e2 = cudaMalloc(&m->sched, 4 * sched.size());
         if (e2 == cudaSuccess) e2 = cudaMemcpy(m->sched, sched.data(), 4 * sched.size(), cudaMemcpyHostToDevice);
         if (e2 != cudaSuccess) {
@@ -1455,23 +1402,13 @@ WsPlan ws_plan(const Layout& L, size_t rhs, bool tc) {
     return w;
 }
 
-// The kernels of an apply of rhs columns: the tensor-memory ones (tc.cu) from
-// three columns on, the column-by-column ones below.  The latter stream and
-// convert every code once per column, the former once per four or eight
-// columns, in steps with a fixed handshake cost.  Whole applies on the device,
-// us, column by column / tensor memory (2-D, leaf 64 unless noted):
-//                        1 column   2          3          4          16
-//   n =  2048 (1-D, 32)  20 / 25    27 / 27    35 / 27    43 / 28    146 / 39
-//   n =  9001 (leaf 32)  43 / 97    77 / 105   112 / 108  150 / 110  526 / 284
-//   n = 16384            43 / 78    75 / 83    115 / 87   153 / 88   556 / 186
-//   n =  8192 (3-D)      54 / 77    95 / 80    138 / 81   179 / 82   644 / 195
-//   n = 32768            81 / 155   146 / -    212 / 177  277 / 179
-// Their workspace must also fit the column-by-column kernels' (which sizes
-// every workspace; V is smaller than B rows wherever a component is read by
-// more than one row tile).
-constexpr size_t kTcColumns = 3;
-bool use_tc(const Layout& L, size_t rhs) {
-    return rhs >= kTcColumns && ws_plan(L, rhs, true).total <= ws_plan(L, rhs, false).total;
+// The kernels of an apply of rhs columns: the tensor-memory ones (tc.cu) where
+// KernelChoice predicts less time for them than for the column-by-column ones
+// below.  Their workspace must also fit the column-by-column kernels' (which
+// sizes every workspace): V has a row for every component, B rows one for every
+// slot, so it does unless the factor arrays hold many components of no block.
+bool use_tc(const qh_matrix* m, size_t rhs) {
+    return m->choice.tensor(rhs) && ws_plan(m->L, rhs, true).total <= ws_plan(m->L, rhs, false).total;
 }
 
 // Workspace of an apply with rhs columns (one column chunk's worth).
@@ -1484,7 +1421,7 @@ int launch_chunk(const qh_matrix* m, const double* x, double* y, size_t rhs, lon
     const Layout& L = m->L;
     const int n = int(L.order);
     auto* w = static_cast<uint8_t*>(ws);
-    const bool tc = use_tc(L, rhs);
+    const bool tc = use_tc(m, rhs);
     const WsPlan P = ws_plan(L, rhs, tc);
     Work W;
     W.xc = reinterpret_cast<double*>(w + P.xc);
