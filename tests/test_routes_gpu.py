@@ -1,4 +1,12 @@
 """Applies of several columns whose structure takes them off the usual path:
+a long 1-D matrix with small leaves, which stays on the column-by-column kernels
+at some column counts and leaves them at others; a row tile whose items have
+more than 32 steps (two runs of step descriptors); matrices of different sizes
+applied at the same time on streams of their own.  Every column equals its own
+one-column apply bit for bit."""
+
+import numpy as np
+import pytest
 
 from qhmat_gb300 import HMatrix
 from qhmat_gb300.construct import spatial_partition
@@ -47,3 +55,32 @@ def _check(h, columns, seed):
 
 def test_long_1d_matrix(cuda_device):
     _check(_points(12001, 1, 16, 6, 1), (2, 3, 4, 5, 8, 9, 17), 2)
+
+
+def test_row_items_of_more_than_32_steps(cuda_device):
+    # 68 blocks of rank 64 beside one tile's rows: 69 k-pairs a split, 35 steps
+    n, c = 64 * 69, range(0, 64 * 69, 64)
+    rng = np.random.default_rng(3)
+    blocks = [(r, r + 64, k, k + 64, 0 if r == k else 64 if r == 0 else 1) for r in c for k in c]
+    _check(_matrix(n, rng.permutation(n), blocks, rng), (3, 4, 5, 9, 17), 4)
+
+
+def test_matrices_at_the_same_time(cuda_device):
+    import torch
+
+    jobs = []
+    for k, (n, dim, leaf, rank, p) in enumerate([(300, 2, 64, 12, 3), (1000, 2, 64, 14, 8), (2049, 1, 32, 6, 4),
+                                                 (3001, 2, 32, 14, 16), (700, 3, 64, 20, 5), (64, 1, 64, 1, 9)]):
+        h = _points(n, dim, leaf, rank, 10 + k)
+        x = torch.from_numpy(np.random.default_rng(20 + k).standard_normal((n, p))).cuda()
+        ws = torch.empty(h.workspace_bytes(p), dtype=torch.uint8, device="cuda")
+        jobs.append((h, x, h.matmul(x), ws, torch.cuda.Stream()))
+    torch.cuda.synchronize()
+    got = [[] for _ in jobs]
+    for _ in range(20):
+        for k, (h, x, _, ws, s) in enumerate(jobs):
+            with torch.cuda.stream(s):
+                got[k].append(h.matmul(x, workspace=ws, check=False))
+    torch.cuda.synchronize()
+    for ys, (_, _, y, _, _) in zip(got, jobs):
+        assert all(torch.equal(y, v) for v in ys)
