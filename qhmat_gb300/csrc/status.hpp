@@ -8,6 +8,8 @@
 
 #include <mutex>
 
+#include "../../include/qhmat_gb300.h"
+
 namespace qhg {
 
 // A handle's words: one per call in flight, up to kKept of them kept for the
@@ -46,7 +48,8 @@ private:
 };
 
 // Run `launch(word)` (returns a QH_* status), wait for the stream and read
-// what the kernels flagged.
+// what the kernels flagged.  A call refused for its arguments has launched
+// nothing and returns at once.
 template <class Launch, class Fail>
 int checked_call(StatusWords& words, cudaStream_t s, Launch&& launch, Fail&& fail) {
     int* word = nullptr;
@@ -54,6 +57,10 @@ int checked_call(StatusWords& words, cudaStream_t s, Launch&& launch, Fail&& fai
     if (e != cudaSuccess) return fail(e, 0);
     *static_cast<volatile int*>(word) = 0;
     const int rc = launch(word);
+    if (rc == QH_EINVAL || rc == QH_EOVERFLOW) {
+        words.give(word);
+        return rc;
+    }
     // (also after a failed launch: kernels before it may still write the word)
     e = cudaStreamSynchronize(s);
     const int st = *static_cast<volatile int*>(word);
