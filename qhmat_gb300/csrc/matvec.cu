@@ -1922,9 +1922,15 @@ int qh_matrix_reconstruct(const qh_matrix* m, double* out, size_t out_count, int
             reconstruct_kernel<<<unsigned(tiles), 128>>>(m->A, n_lr, nb, d_blocks, left, right, int(n), d_out);
             e = cudaGetLastError();
         }
-        // (host memory only; while the device works.  Before the allocation, its
-        // mappings and the page faults held each other up: 1.4 ms more.)
-        PagePopulator(out_on_device ? nullptr : out, 8 * n * n).wait();
+        // (while the device works.  Before the allocation, its mappings and the
+        // page faults held each other up: 1.4 ms more.  Only pageable memory, whose
+        // pages may be absent, and only if the copy will follow: a pointer that
+        // the host may not touch is the copy's to judge.)
+        if (e == cudaSuccess && !out_on_device) {
+            cudaPointerAttributes at{};
+            if (cudaPointerGetAttributes(&at, out) != cudaSuccess) cudaGetLastError();
+            else if (at.type == cudaMemoryTypeUnregistered) PagePopulator(out, 8 * n * n).wait();
+        }
         if (e == cudaSuccess)
             e = out_on_device ? cudaDeviceSynchronize() : cudaMemcpy(out, d_out, 8 * n * n, cudaMemcpyDeviceToHost);
         return e == cudaSuccess ? QH_OK : cuda_fail(e, "reconstruct");
