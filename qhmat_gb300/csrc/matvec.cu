@@ -924,19 +924,11 @@ __global__ void __launch_bounds__(64) combine_kernel(Arena A, Work W, double* __
 // Decode every code from the resident layout through the same fragment
 // routines the apply kernels feed to the MMA (group_digits uses the permutes
 // and masks of group_mma).  out[comp_base[c] + i] = code i of component c
-// (i: block column on the right side, clustered row on the left), as it is or
-// as a factor entry (FP64, times the component's scale).
-__device__ __forceinline__ void put_code(int* out, long long i, long long code, const double*, int) {
-    out[i] = int(code);
-}
-__device__ __forceinline__ void put_code(double* out, long long i, long long code, const double* scale, int c) {
-    out[i] = __dmul_rn(double(code), scale[c]);
-}
+// (i: block column on the right side, clustered row on the left).
 
 // Part y of gridDim.y: chunks of a task.
-template <class Out>
 __device__ __forceinline__ void decode_col(const Arena& A, int n_tasks, int block, int blocks,
-                                           const long long* __restrict__ comp_base, Out* out) {
+                                           const long long* __restrict__ comp_base, int* out) {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int warps = blocks * (blockDim.x >> 5);
     for (int ti = block * (blockDim.x >> 5) + (threadIdx.x >> 5); ti < n_tasks; ti += warps) {
@@ -966,7 +958,7 @@ __device__ __forceinline__ void decode_col(const Arena& A, int n_tasks, int bloc
                     const int c = A.task_rec[T.comp_idx + j].comp;
                     for (int k = 0; k < 8; ++k) {
                         const int i = ch * kColChunk + slot_entry(k >> 2, k & 3, t);
-                        if (i < T.n) put_code(out, comp_base[c] + i, int64_t(u[hh][k]) - (int64_t(1) << (T.width - 1)), A.comp_sr, c);
+                        if (i < T.n) out[comp_base[c] + i] = int(int64_t(u[hh][k]) - (int64_t(1) << (T.width - 1)));
                     }
                 }
             }
@@ -976,9 +968,8 @@ __device__ __forceinline__ void decode_col(const Arena& A, int n_tasks, int bloc
 
 // Part y of gridDim.y: a run of a unit's k-pairs (found by summing the bytes of
 // those before it).
-template <class Out>
 __device__ __forceinline__ void decode_row(const Arena& A, int n_units, int block, int blocks,
-                                           const long long* __restrict__ comp_base, Out* out) {
+                                           const long long* __restrict__ comp_base, int* out) {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int warps = blocks * (blockDim.x >> 5);
     for (int ui = block * (blockDim.x >> 5) + (threadIdx.x >> 5); ui < n_units; ui += warps) {
@@ -1012,7 +1003,7 @@ __device__ __forceinline__ void decode_row(const Arena& A, int n_units, int bloc
                     const int e = slot_entry(k >> 2, k & 3, t);
                     const int c = A.slot_rec[U.slot0 + 32 * i + e].comp;
                     if (c < 0) continue;
-                    put_code(out, comp_base[c] + T.row0 + tr, u[hh][k], A.comp_sl, c);
+                    out[comp_base[c] + T.row0 + tr] = int(u[hh][k]);
                 }
             }
         }
@@ -1020,18 +1011,16 @@ __device__ __forceinline__ void decode_row(const Arena& A, int n_units, int bloc
 }
 
 // Blocks [0, col_blocks) of x decode the column side, the others the row side.
-template <class Out>
-__global__ void decode_kernel(Arena A, int n_tasks, int col_blocks, const long long* rbase, Out* rout, int n_units,
-                              const long long* lbase, Out* lout) {
+__global__ void decode_kernel(Arena A, int n_tasks, int col_blocks, const long long* rbase, int* rout, int n_units,
+                              const long long* lbase, int* lout) {
     if (int(blockIdx.x) < col_blocks) decode_col(A, n_tasks, blockIdx.x, col_blocks, rbase, rout);
     else decode_row(A, n_units, int(blockIdx.x) - col_blocks, int(gridDim.x) - col_blocks, lbase, lout);
 }
-template <class Out>
-cudaError_t launch_decode(const Arena& A, int n_tasks, const long long* rbase, Out* rout, int n_units,
-                          const long long* lbase, Out* lout) {
+cudaError_t launch_decode(const Arena& A, int n_tasks, const long long* rbase, int* rout, int n_units,
+                          const long long* lbase, int* lout) {
     const int cb = std::min((n_tasks + 7) / 8, 4096), rb = std::min((n_units + 7) / 8, 4096);
     if (cb + rb == 0) return cudaSuccess;
-    decode_kernel<Out><<<dim3(unsigned(cb + rb), 8), 256>>>(A, n_tasks, cb, rbase, rout, n_units, lbase, lout);
+    decode_kernel<<<dim3(unsigned(cb + rb), 8), 256>>>(A, n_tasks, cb, rbase, rout, n_units, lbase, lout);
     return cudaGetLastError();
 }
 
@@ -1056,14 +1045,21 @@ __global__ void factor_base_kernel(Arena A, int n_lr, const DenseOut* blocks, lo
 // out[perm[row] * n + perm[col]].
 //
 // Bound by the FP64 unit: one multiply and one add per component and entry (the
-// factors are scaled once, by decode_kernel; scaling them per entry took six
-// operations).  One block per 32 x 32 tile, factors 16 components at a time in
-// shared memory, 2 x 4 entries a thread.  n = 2048, 2-D, 11587 components:
-// 657 -> 250 us (about 180 us by the rate of the FP64 unit).
+// codes are scaled as they enter a tile, 6 % of its operations; scaling them per
+// entry took six each).  One block per 32 x 32 tile, factors 16 components at a
+// time in shared memory, 2 x 4 entries a thread.  n = 2048, 2-D, 11587
+// components: 657 -> 250 us (about 180 us by the rate of the FP64 unit).  Factors
+// scaled by decode_kernel took the same time (device call 412 us, now 410; 5000
+// unknowns 2150, now 2213) but twice the scratch.
 constexpr int kDenseTile = 32, kDenseComps = 16;
+// A code as a double: its bits below those of 1.5 2^52, minus that number (one
+// exact FP64 operation, at twice the rate of a conversion).
+__device__ __forceinline__ double code_value(int c) {
+    return __dsub_rn(__longlong_as_double(0x4338000000000000LL + c), 6755399441055744.0);
+}
 __global__ void __launch_bounds__(128) reconstruct_kernel(Arena A, int n_lr, int nb, const DenseOut* __restrict__ blocks,
-                                                          const double* __restrict__ left,
-                                                          const double* __restrict__ right, int n,
+                                                          const int* __restrict__ left,
+                                                          const int* __restrict__ right, int n,
                                                           double* __restrict__ out) {
     __shared__ double P[kDenseComps][kDenseTile], Q[kDenseComps][kDenseTile];
     int lo = 0, hi = nb - 1;
@@ -1092,8 +1088,13 @@ __global__ void __launch_bounds__(128) reconstruct_kernel(Arena A, int n_lr, int
         for (int j0 = 0; j0 < d.rank; j0 += kDenseComps) {
             const int jn = min(kDenseComps, d.rank - j0);
             for (int j = ty; j < jn; j += 4) {
-                P[j][tx] = i0 + tx < d.m ? left[B.left + (long long)(j0 + j) * d.m + i0 + tx] : 0.0;
-                Q[j][tx] = k0 + tx < d.n ? right[B.right + (long long)(j0 + j) * d.n + k0 + tx] : 0.0;
+                const int c = d.comp0 + j0 + j;
+                P[j][tx] = i0 + tx < d.m ? __dmul_rn(code_value(left[B.left + (long long)(j0 + j) * d.m + i0 + tx]),
+                                                     __ldg(A.comp_sl + c))
+                                         : 0.0;
+                Q[j][tx] = k0 + tx < d.n ? __dmul_rn(code_value(right[B.right + (long long)(j0 + j) * d.n + k0 + tx]),
+                                                     __ldg(A.comp_sr + c))
+                                         : 0.0;
             }
             __syncthreads();
             for (int j = 0; j < jn; ++j) {
@@ -1890,7 +1891,7 @@ int qh_matrix_reconstruct(const qh_matrix* m, double* out, size_t out_count, int
         if (tiles > INT32_MAX) return fail(QH_EOVERFLOW, "CUDA launch grid too large");
         // one allocation (separate ones were slower at every order): factors,
         // bases, blocks, and the output if on the host
-        const size_t parts[5] = {8 * size_t(ltotal), 8 * size_t(rtotal), 16 * size_t(m->L.n_comp),
+        const size_t parts[5] = {4 * size_t(ltotal), 4 * size_t(rtotal), 16 * size_t(m->L.n_comp),
                                  sizeof(DenseOut) * size_t(nb), out_on_device ? 0 : 8 * n * n};
         size_t at[5], bytes = 0;
         for (int i = 0; i < 5; ++i) {
@@ -1904,8 +1905,8 @@ int qh_matrix_reconstruct(const qh_matrix* m, double* out, size_t out_count, int
             }
         } buf;
         if (cudaMalloc(&buf.p, bytes) != cudaSuccess) return fail(QH_ERUNTIME, "cudaMalloc: out of device memory");
-        auto* left = reinterpret_cast<double*>(buf.p + at[0]);
-        auto* right = reinterpret_cast<double*>(buf.p + at[1]);
+        auto* left = reinterpret_cast<int*>(buf.p + at[0]);
+        auto* right = reinterpret_cast<int*>(buf.p + at[1]);
         auto* lb = reinterpret_cast<long long*>(buf.p + at[2]);
         auto* rb = lb + m->L.n_comp;
         auto* d_blocks = reinterpret_cast<DenseOut*>(buf.p + at[3]);
@@ -1916,7 +1917,7 @@ int qh_matrix_reconstruct(const qh_matrix* m, double* out, size_t out_count, int
         if (e == cudaSuccess && area < n * n) e = cudaMemsetAsync(d_out, 0, 8 * n * n, nullptr);
         if (e == cudaSuccess && n_lr) {
             factor_base_kernel<<<unsigned(n_lr), 32>>>(m->A, n_lr, d_blocks, lb, rb);
-            e = launch_decode<double>(m->A, m->L.n_tasks, rb, right, m->L.n_units, lb, left);
+            e = launch_decode(m->A, m->L.n_tasks, rb, right, m->L.n_units, lb, left);
         }
         if (e == cudaSuccess && tiles) {
             reconstruct_kernel<<<unsigned(tiles), 128>>>(m->A, n_lr, nb, d_blocks, left, right, int(n), d_out);
@@ -1975,7 +1976,7 @@ int qh_debug_decode(const qh_matrix* m, int side, int32_t* out, size_t out_count
         int rc = QH_OK;
         e = cudaMemcpy(d_off, off.data(), sizeof(long long) * off.size(), cudaMemcpyHostToDevice);
         if (e == cudaSuccess) {
-            e = launch_decode<int>(m->A, side == 1 ? m->L.n_tasks : 0, d_off, d_out, side == 0 ? m->L.n_units : 0, d_off,
+            e = launch_decode(m->A, side == 1 ? m->L.n_tasks : 0, d_off, d_out, side == 0 ? m->L.n_units : 0, d_off,
                                    d_out);
         }
         if (e == cudaSuccess) e = cudaMemcpy(out, d_out, sizeof(int) * total, cudaMemcpyDeviceToHost);
