@@ -362,6 +362,8 @@ QH_API int qh_batch_scatter(const qh_batch_entry* table, size_t count, int P, co
  * is issued -- and records the timeout in a status int exactly as the apply
  * kernels do; returns QH_ERUNTIME "device copy wait timed out" when the bit
  * came back (the expected outcome), QH_OK if the wait unexpectedly succeeded.
+ * A second kernel does the same with the tensor-memory kernels' wait, and a warp
+ * beside it must end when its block gives up (QH_ECUDA otherwise).
  * No reference counterpart. */
 QH_API int qh_debug_wait_timeout(int device, int polls);
 

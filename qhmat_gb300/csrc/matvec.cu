@@ -1843,19 +1843,26 @@ int qh_debug_wait_timeout(int device, int polls) {
     int rc = check_device(device);
     if (rc) return rc;
     DeviceGuard g(device);
+    // status words: the streaming kernels' wait, the two warps of the
+    // tensor-memory kernels'; then which lanes of those gave up
+    constexpr int kWords = 3 + 64;
     int* d = nullptr;
-    cudaError_t e = cudaMalloc(&d, sizeof(int));
+    cudaError_t e = cudaMalloc(&d, kWords * sizeof(int));
     if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc");
-    int h = 0;
-    e = cudaMemset(d, 0, sizeof(int));
+    int h[kWords] = {};
+    e = cudaMemset(d, 0, kWords * sizeof(int));
     if (e == cudaSuccess) {
         wait_timeout_kernel<<<1, 32>>>(polls, d);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaMemcpy(&h, d, sizeof(int), cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = tc_debug_give_up(polls, d + 1, d + 3);
+    if (e == cudaSuccess) e = cudaMemcpy(h, d, sizeof(h), cudaMemcpyDeviceToHost);
     cudaFree(d);
     if (e != cudaSuccess) return cuda_fail(e, "debug wait");
-    if (h & kStatusTimeout) return fail(QH_ERUNTIME, "device copy wait timed out");
+    // (the warp that was told to give up has not run out of its own tests)
+    if (std::count(h + 3, h + kWords, 1) != 64 || h[1] != kStatusTimeout || h[2] != 0)
+        return fail(QH_ECUDA, "a block did not give up as a whole");
+    if (h[0] & kStatusTimeout) return fail(QH_ERUNTIME, "device copy wait timed out");
     return QH_OK;
 }
 

@@ -530,7 +530,7 @@ __global__ void __launch_bounds__(ColRoles::kThreads, 1) pf_column_kernel(Arena 
                 for (int m = 0; m < I.planes; ++m, ++ai) {
                     if (ai % kConvGroups != group) continue;
                     const int sa = ai % kAStages;
-                    ok = wait_bar(&S.a_full[sa], (ai / kAStages) & 1, abort_flag, status);
+                    ok = warp_wait(&S.a_full[sa], (ai / kAStages) & 1, abort_flag, status);
                     if (!ok) break;
                     convert_plane<kGroupWarps * 32>(sm + kOffARaw + sa * kPfPlaneBytes, sm + kOffAF16 + sa * kPfTileBytes,
                                                     m, I.planes, 0, 0, ctid);
@@ -570,7 +570,7 @@ __global__ void __launch_bounds__(ColRoles::kThreads, 1) pf_column_kernel(Arena 
             for (int r = 0; r < 32; ++r) t[r] = 0.0f;
             for (int kc0 = 0; kc0 < I.nkc; kc0 += kSegChunks, ++seg) {
                 const int buf = seg & 1;
-                if (!(ok = wait_bar(&S.acc_full[buf], (seg >> 1) & 1, abort_flag, status))) break;
+                if (!(ok = warp_wait(&S.acc_full[buf], (seg >> 1) & 1, abort_flag, status))) break;
                 tc_fence_after();
                 const uint32_t base = tmem + (uint32_t(32 * q) << 16) + uint32_t(buf * kAccStride);
 #pragma unroll
@@ -774,7 +774,7 @@ __global__ void __launch_bounds__(RowRoles::kThreads, 1) pf_row_kernel(Arena A, 
                 const PfRowChunk C = A.chunks[I.chunk0 + c];
                 if (c + 2 < I.nchunks) prefetch_l1(A.chunks + I.chunk0 + c + 2);
                 const int sb = bi % kBStages;
-                ok = wait_bar(&S.b_full[sb], (bi / kBStages) & 1, abort_flag, status);
+                ok = warp_wait(&S.b_full[sb], (bi / kBStages) & 1, abort_flag, status);
                 if (!ok) break;
                 if (C.kind == 0)
                     convert_u<kGroupWarps * 32>(reinterpret_cast<const float*>(sm + kOffBRaw + sb * kURawBytes),
@@ -801,7 +801,7 @@ __global__ void __launch_bounds__(RowRoles::kThreads, 1) pf_row_kernel(Arena A, 
                 for (int m = 0; m < nt; ++m, ++ai) {
                     if (ai % kConvGroups != group) continue;
                     const int sa = ai % kAStages;
-                    ok = wait_bar(&S.a_full[sa], (ai / kAStages) & 1, abort_flag, status);
+                    ok = warp_wait(&S.a_full[sa], (ai / kAStages) & 1, abort_flag, status);
                     if (!ok) break;
                     if (C.kind == 0) {
                         const uint8_t* raw = sm + kOffARaw + sa * kPfPlaneBytes;
@@ -851,7 +851,7 @@ __global__ void __launch_bounds__(RowRoles::kThreads, 1) pf_row_kernel(Arena A, 
                 while (c_end < I.nchunks && c_end - c < kSegChunks && A.chunks[I.chunk0 + c_end].kind == kind) ++c_end;
                 c = c_end;
                 const int buf = seg & 1;
-                if (!(ok = wait_bar(&S.acc_full[buf], (seg >> 1) & 1, abort_flag, status))) break;
+                if (!(ok = warp_wait(&S.acc_full[buf], (seg >> 1) & 1, abort_flag, status))) break;
                 ++seg;
                 tc_fence_after();
                 const uint32_t base = tmem + (uint32_t(32 * q) << 16) + uint32_t(buf * kAccStride);

@@ -541,11 +541,11 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (unsigned ri = unsigned(wg - 1);; ri += 2) {
             const int s = ri % kStages;
             const unsigned ph = (ri / kStages) & 1;
-            if (!wait_bar(&S.raw_full[s], ph, abort_flag, status)) break;
+            if (!warp_wait(&S.raw_full[s], ph, abort_flag, status)) break;
             const unsigned used = ri - M::kAStages;  // the step whose A stage this one takes
             const uint32_t word = *reinterpret_cast<volatile uint32_t*>(&S.step[ri % (2 * kStages)]);
             const int info = *reinterpret_cast<volatile int*>(&S.task[s][sub]);
-            if (ri >= M::kAStages && !wait_bar(&S.done[used % kStages], (used / kStages) & 1, abort_flag, status)) break;
+            if (ri >= M::kAStages && !warp_wait(&S.done[used % kStages], (used / kStages) & 1, abort_flag, status)) break;
             if (word != kNoMore) {
                 // (rows past the task's components convert whatever bytes are
                 // there: finite values in accumulator rows that nothing reads)
@@ -616,7 +616,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 for (int t = 0; t < 4; ++t) v[r][t] = 0;
             for (bool end = false; !end; ++seg) {
                 const int buf = seg & 1;
-                ok = wait_bar(&S.acc_full[buf], (seg >> 1) & 1, abort_flag, status);
+                ok = warp_wait(&S.acc_full[buf], (seg >> 1) & 1, abort_flag, status);
                 if (!ok) break;
                 __syncwarp();
                 tc_fence_after();
@@ -903,10 +903,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (unsigned ri = unsigned(wg - 1);; ri += 2) {
             const int s = ri % kStages;
             const unsigned ph = (ri / kStages) & 1;
-            if (!wait_bar(&S.raw_full[s], ph, abort_flag, status)) break;
+            if (!warp_wait(&S.raw_full[s], ph, abort_flag, status)) break;
             const unsigned used = ri - M::kAStages;  // the step whose A stage this one takes
             const uint32_t word = *reinterpret_cast<volatile uint32_t*>(&S.step[ri % (2 * kStages)]);
-            if (ri >= M::kAStages && !wait_bar(&S.done[used % kStages], (used / kStages) & 1, abort_flag, status)) break;
+            if (ri >= M::kAStages && !warp_wait(&S.done[used % kStages], (used / kStages) & 1, abort_flag, status)) break;
             if (word != kNoMore) {
                 const int wide = int(word >> 24) & 1;  // 1: 64 tile rows x 2 planes, 0: 32 x 4
                 const int m0 = row >> (5 + wide), tr = row & (31 + 32 * wide), rr = tr & 15;
@@ -963,7 +963,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             weights = 0;
             for (bool end = false; !end; ++seg) {
                 const int buf = seg & 1;
-                ok = wait_bar(&S.acc_full[buf], (seg >> 1) & 1, abort_flag, status);
+                ok = warp_wait(&S.acc_full[buf], (seg >> 1) & 1, abort_flag, status);
                 if (!ok) break;
                 __syncwarp();
                 tc_fence_after();
@@ -1061,7 +1061,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (i >= 0) {
                 if (q[0] < 0) break;
                 const int sb = bi % kStages;
-                if (bi >= kStages) ok = wait_bar(&S.done[sb], ((bi / kStages) - 1) & 1, abort_flag, status);
+                if (bi >= kStages) ok = warp_wait(&S.done[sb], ((bi / kStages) - 1) & 1, abort_flag, status);
                 if (!ok) break;
                 uint8_t* dst = sm + M::kOffB + sb * C::kB + pair * 2 * C::kBCol + slot0 * 16;
 #pragma unroll
@@ -1094,6 +1094,22 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
     tc_fence_after();
     if (warp == 1) tmem_free(tmem, 512);
+}
+
+// Test aid: warp 0 waits for a phase that nothing completes, `polls` tests at
+// most, and tells the block; warp 1 waits for another and ends when told.  out: 1
+// for each lane that gave up.
+__global__ void __launch_bounds__(64) give_up_kernel(int polls, int* status, int* out) {
+    __shared__ uint64_t bar[2];
+    __shared__ int abort_flag;
+    const int warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 2; ++i) mbar_init(&bar[i], 1);
+        abort_flag = 0;
+    }
+    __syncthreads();
+    const bool ok = warp_wait(&bar[warp], 0, &abort_flag, status + warp, warp ? kWaitLimit : polls);
+    out[threadIdx.x] = ok ? 0 : 1;
 }
 
 // ------------------------------------------------------------------ combine
@@ -1162,6 +1178,11 @@ cudaError_t tc_setup() {
     if (e == cudaSuccess) e = allow_smem(tc_row_kernel<4>, RowSmem<4>::kBytes);
     if (e == cudaSuccess) e = allow_smem(tc_row_kernel<8>, RowSmem<8>::kBytes);
     return e;
+}
+
+cudaError_t tc_debug_give_up(int polls, int* status, int* out) {
+    tc::give_up_kernel<<<1, 64>>>(polls, status, out);
+    return cudaGetLastError();
 }
 
 cudaError_t tc_launch(const TcArgs& a, cudaStream_t s, void (*mark)(void*, int), void* ctx) {

@@ -21,4 +21,8 @@ cudaError_t tc_setup();
 // called after the column kernel.
 cudaError_t tc_launch(const TcArgs& a, cudaStream_t s, void (*mark)(void*, int), void* ctx);
 
+// Test aid (qh_debug_wait_timeout): two warps whose waits nothing ends; status: two
+// words, out: 64.
+cudaError_t tc_debug_give_up(int polls, int* status, int* out);
+
 }  // namespace qhg

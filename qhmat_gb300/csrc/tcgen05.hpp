@@ -52,6 +52,24 @@ __device__ __forceinline__ bool wait_bar(uint64_t* bar, unsigned parity, volatil
     if (mbar_try(bar, parity)) return true;
     return wait_bar_slow(bar, parity, abort_flag, status);
 }
+// The same for a whole warp that goes on with warp-wide instructions: its lanes
+// agree at every test.  A lane that gave up while others went on would leave them
+// waiting for it at the next of those instructions, without a limit.
+__device__ __forceinline__ bool warp_wait_slow(uint64_t* bar, unsigned parity, volatile int* abort_flag, int* status,
+                                               int limit) {
+    for (int i = 0; i < limit; ++i) {
+        if (__all_sync(0xFFFFFFFFu, mbar_try(bar, parity))) return true;
+        if ((i & 255) == 255 && __any_sync(0xFFFFFFFFu, *abort_flag)) return false;
+    }
+    *abort_flag = 1;
+    if (status) atomicOr(status, kStatusTimeout);
+    return false;
+}
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, unsigned parity, volatile int* abort_flag, int* status,
+                                          int limit = kWaitLimit) {
+    if (__all_sync(0xFFFFFFFFu, mbar_try(bar, parity))) return true;
+    return warp_wait_slow(bar, parity, abort_flag, status, limit);
+}
 // Pull a descriptor two items (chunks) ahead into L1, so that the roles that
 // read it find it there instead of waiting for L2 at every item.
 __device__ __forceinline__ void prefetch_l1(const void* ptr) {
