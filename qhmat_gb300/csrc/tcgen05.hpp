@@ -8,6 +8,8 @@
 #include <cstdint>
 
 #include "../../include/qhmat_gb300.h"
+#include "pdl.hpp"
+#include "waits.hpp"
 
 namespace qhg {
 namespace tc {
@@ -35,40 +37,33 @@ __device__ __forceinline__ bool mbar_try(uint64_t* bar, unsigned parity) {
         : "memory");
     return ok != 0;
 }
-// Bounded wait; gives up when the block has been told to abort, or after
-// kWaitLimit tests (then it raises the abort flag and the timeout bit).  The
-// first test stands alone, outside the loop and the bookkeeping of giving up: a
-// wait for a phase that has completed then takes ~20 cycles instead of ~200.
-__device__ __forceinline__ bool wait_bar_slow(uint64_t* bar, unsigned parity, volatile int* abort_flag, int* status) {
-    for (int i = 0; i < kWaitLimit; ++i) {
-        if (mbar_try(bar, parity)) return true;
-        if ((i & 255) == 255 && *abort_flag) return false;
+// Bounded wait (waits.hpp): giving up tells the block and, unless that was told
+// already, raises the timeout bit.  The first test stands alone, outside the loop
+// and the bookkeeping of giving up: a wait for a phase that has completed then
+// takes ~20 cycles instead of ~200.
+__device__ __forceinline__ bool gave_up(Waited w, volatile int* abort_flag, int* status) {
+    if (w == Waited::kRanOut) {
+        *abort_flag = 1;
+        if (status) atomicOr(status, kStatusTimeout);
     }
-    *abort_flag = 1;
-    if (status) atomicOr(status, kStatusTimeout);
-    return false;
+    return w != Waited::kDone;
 }
 __device__ __forceinline__ bool wait_bar(uint64_t* bar, unsigned parity, volatile int* abort_flag, int* status) {
     if (mbar_try(bar, parity)) return true;
-    return wait_bar_slow(bar, parity, abort_flag, status);
+    const Waited w = bounded_wait([&] { return mbar_try(bar, parity); }, [&] { return *abort_flag != 0; },
+                                  [] { pdl_wait(); }, kWaitLimit);
+    return !gave_up(w, abort_flag, status);
 }
 // The same for a whole warp that goes on with warp-wide instructions: its lanes
 // agree at every test.  A lane that gave up while others went on would leave them
 // waiting for it at the next of those instructions, without a limit.
-__device__ __forceinline__ bool warp_wait_slow(uint64_t* bar, unsigned parity, volatile int* abort_flag, int* status,
-                                               int limit) {
-    for (int i = 0; i < limit; ++i) {
-        if (__all_sync(0xFFFFFFFFu, mbar_try(bar, parity))) return true;
-        if ((i & 255) == 255 && __any_sync(0xFFFFFFFFu, *abort_flag)) return false;
-    }
-    *abort_flag = 1;
-    if (status) atomicOr(status, kStatusTimeout);
-    return false;
-}
 __device__ __forceinline__ bool warp_wait(uint64_t* bar, unsigned parity, volatile int* abort_flag, int* status,
                                           int limit = kWaitLimit) {
-    if (__all_sync(0xFFFFFFFFu, mbar_try(bar, parity))) return true;
-    return warp_wait_slow(bar, parity, abort_flag, status, limit);
+    const unsigned all = 0xFFFFFFFFu;
+    if (__all_sync(all, mbar_try(bar, parity))) return true;
+    const Waited w = bounded_wait([&] { return __all_sync(all, mbar_try(bar, parity)) != 0; },
+                                  [&] { return __any_sync(all, *abort_flag) != 0; }, [] { pdl_wait(); }, limit);
+    return !gave_up(w, abort_flag, status);
 }
 // Pull a descriptor two items (chunks) ahead into L1, so that the roles that
 // read it find it there instead of waiting for L2 at every item.
