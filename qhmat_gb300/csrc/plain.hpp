@@ -155,15 +155,17 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, unsigned parity) {
         : "memory");
     return ok != 0;
 }
-// Bounded wait: gives up (returns false) after `limit` tests (kWaitLimit:
-// seconds at most) instead of hanging; callers record the failure in the
+// Bounded wait: gives up (returns false) after `limit` tests (kWaitLimit: about
+// 16 seconds) instead of hanging; callers record the failure in the
 // status word, stop issuing copies, give the copies already issued one more
 // bounded wait each and return (best effort: a copy still outstanding after
-// that wait is abandoned with the block).
+// that wait is abandoned with the block).  Of a whole warp, whose lanes agree at
+// every test: a lane that gave up alone would leave the others waiting for it at
+// their next warp-wide instruction, without a limit.
 constexpr int kWaitLimit = 1 << 22;
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity, int limit = kWaitLimit) {
     for (int i = 0; i < limit; ++i)
-        if (mbar_try_wait(bar, parity)) return true;
+        if (__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;
     return false;
 }
 // Order this thread's (and, after a warp barrier, its warp's) earlier generic
