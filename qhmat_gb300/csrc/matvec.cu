@@ -1287,13 +1287,8 @@ int upload(Layout&& L, int device, qh_matrix** out) {
         delete m;
         return cuda_fail(e, "cudaMemcpy host-to-device");
     }
-    {
-        int* word = nullptr;  // the first status word (more only for calls at the same time)
-        e = m->words.take(&word);
-        if (e == cudaSuccess) m->words.give(word);
-    }
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowPipeSmem);
+    m->words.prepare();
+    e = cudaFuncSetAttribute(row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowPipeSmem);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(column_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kColPipeSmem);
     if (e == cudaSuccess) e = tc_setup();
@@ -1695,8 +1690,8 @@ int qh_matmul_device_checked(const qh_matrix* m, const double* x, double* y, siz
     return checked_call(
         const_cast<qh_matrix*>(m)->words, static_cast<cudaStream_t>(stream),
         [&](int* word) { return qh_matmul_device(m, x, y, rhs, workspace, workspace_bytes, stream, word); },
-        [](cudaError_t e, int st) {
-            if (e != cudaSuccess) return cuda_fail(e, "CUDA kernel execution");
+        [](cudaError_t e, int st, const char* what) {
+            if (e != cudaSuccess) return cuda_fail(e, what);
             if (st & kStatusNonfinite) return fail(QH_EINVAL, "nonfinite right-hand side");
             return fail(QH_ERUNTIME, "device copy wait timed out");
         });

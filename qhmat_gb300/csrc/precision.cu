@@ -1149,15 +1149,7 @@ int pf_upload(const HostMatrix& hm, int device, int grid, double row_items_per_c
         delete m;
         return cuda_err(e, "precision form upload");
     }
-    {
-        int* word = nullptr;  // the first status word (more only for calls at the same time)
-        e = m->words.take(&word);
-        if (e != cudaSuccess) {
-            delete m;
-            return cuda_err(e, "cudaMallocHost");
-        }
-        m->words.give(word);
-    }
+    m->words.prepare();
     std::vector<uint8_t>().swap(m->L.arena);
     const PfSections& S = m->L.sec;
     auto* b = static_cast<const uint8_t*>(m->arena);
@@ -1304,8 +1296,8 @@ int qh_pmatmul_device_checked(const qh_pmatrix* m, const double* x, double* y, s
     return checked_call(
         const_cast<qh_pmatrix*>(m)->words, static_cast<cudaStream_t>(stream),
         [&](int* word) { return qh_pmatmul_device(m, x, y, rhs, workspace, workspace_bytes, stream, word); },
-        [](cudaError_t e, int st) {
-            if (e != cudaSuccess) return cuda_err(e, "CUDA kernel execution");
+        [](cudaError_t e, int st, const char* what) {
+            if (e != cudaSuccess) return cuda_err(e, what);
             if (st & QH_STATUS_NONFINITE) return set_error(QH_EINVAL, "nonfinite right-hand side");
             return set_error(QH_ERUNTIME, "device copy wait timed out");
         });

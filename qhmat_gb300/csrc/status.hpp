@@ -19,6 +19,13 @@ public:
     ~StatusWords() {
         for (int i = 0; i < n_; ++i) cudaFreeHost(idle_[i]);
     }
+    // The first word, ahead of the first call (calls at the same time make more).
+    // Without memory for it now, that call asks again.
+    void prepare() {
+        int* word = nullptr;
+        if (take(&word) == cudaSuccess) give(word);
+        else cudaGetLastError();
+    }
     cudaError_t take(int** out) {
         {
             std::lock_guard<std::mutex> lock(mu_);
@@ -48,13 +55,13 @@ private:
 };
 
 // Run `launch(word)` (returns a QH_* status), wait for the stream and read
-// what the kernels flagged.  A call refused for its arguments has launched
+// what the kernels flagged (fail(error, status bits, what failed)).  A call refused for its arguments has launched
 // nothing and returns at once.
 template <class Launch, class Fail>
 int checked_call(StatusWords& words, cudaStream_t s, Launch&& launch, Fail&& fail) {
     int* word = nullptr;
     cudaError_t e = words.take(&word);
-    if (e != cudaSuccess) return fail(e, 0);
+    if (e != cudaSuccess) return fail(e, 0, "cudaMallocHost");
     *static_cast<volatile int*>(word) = 0;
     const int rc = launch(word);
     if (rc == QH_EINVAL || rc == QH_EOVERFLOW) {
@@ -66,7 +73,7 @@ int checked_call(StatusWords& words, cudaStream_t s, Launch&& launch, Fail&& fai
     const int st = *static_cast<volatile int*>(word);
     words.give(word);
     if (rc) return rc;
-    if (e != cudaSuccess || st) return fail(e, st);
+    if (e != cudaSuccess || st) return fail(e, st, "CUDA kernel execution");
     return 0;
 }
 
