@@ -186,11 +186,13 @@ class BatchedHMatrices:
             if autotune:
                 params = self._autotune(pf_idx, images, cache)
             self.batches.append(self._make(images, pf_idx, True, seg=self.pf_seg, **params))
-        # plain matrices in sub-batches by right-hand-side count: the plain
-        # form's work grows with the columns it is given (every matrix of a
-        # sub-batch is applied to its widest column count), so a 3-column
-        # matrix should not ride in a 32-column operand; these edges pad
-        # uniform 1..32-column requests by ~14% (4/8/16/32 edges: ~30%)
+        # plain matrices in sub-batches by right-hand-side count: every matrix
+        # of a sub-batch is applied to its widest column count, and the plain
+        # form's work grows with the columns it is given (one by one on the
+        # column-by-column kernels, in groups of eight on the others), so a
+        # 3-column matrix should not ride in a 32-column operand.  The edges
+        # pad uniform 1..32-column requests by ~14% counted in columns
+        # (4/8/16/32 edges: ~30%)
         edges = (0, 2, 4, 6, 8, 12, 16, 24, 32, 1 << 30)
         for lo, hi in zip(edges[:-1], edges[1:]):
             sub = [k for k in pl_idx if lo < self.rhs[k] <= hi]

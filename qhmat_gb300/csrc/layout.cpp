@@ -829,8 +829,6 @@ Layout build_layout(const HostMatrix& m) {
     S.iperm = place(4 * m.order);  // source index -> clustered position
     S.lr = place(sizeof(LowRankDesc) * lr.size());
     S.dd = place(sizeof(DenseDesc) * dd.size());
-    S.comp_w = place(C);
-    S.comp_s = place(8 * C);
     S.tasks = place(sizeof(ColTask) * tasks.size());
     S.task_rec = place(sizeof(TaskRec) * task_rec.size());
     S.qcodes = place(qcodes.size() + 16);
@@ -861,10 +859,6 @@ Layout build_layout(const HostMatrix& m) {
     if (!lr.empty()) std::memcpy(at<LowRankDesc>(A, S.lr), lr.data(), sizeof(LowRankDesc) * lr.size());
     if (!dd.empty()) std::memcpy(at<DenseDesc>(A, S.dd), dd.data(), sizeof(DenseDesc) * dd.size());
     for (size_t c = 0; c < C; ++c) {
-        at<uint8_t>(A, S.comp_w)[c] = m.width[c];
-        // One rounding: s_P * s_Q.  In exact arithmetic the block contribution
-        // sum_j (s_P c_P)(sum_k s_Q c_Q x) equals sum_j c_P (s_P s_Q) sum_k c_Q x.
-        at<double>(A, S.comp_s)[c] = m.left_scale[c] * m.right_scale[c];
         at<double>(A, S.comp_sl)[c] = m.left_scale[c];
         at<double>(A, S.comp_sr)[c] = m.right_scale[c];
     }

@@ -36,8 +36,10 @@
 // The only rounding steps are the fixed-point conversions of x and u (2^-63
 // of the column's largest |x|, ~2^-62 of the component's and of the tile's
 // bound on |u|), the product s^P s^Q, and the final FP64 conversions: the
-// result agrees with the
-// reference's FP64 matmul (src/qhmat/core.cpp:360-390) to ~1e-15 in norm.
+// result agrees with the reference's FP64 matmul (src/qhmat/core.cpp:360-390) to
+// ~1e-15 in norm.  (Less for a tile that mixes very narrow and very wide codes of
+// equal size, which an allocation of widths by singular value never makes: a
+// 32-bit component's u is 2^-29 of a 3-bit one's there, and keeps 33 bits.)
 #include <cooperative_groups.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -1311,8 +1313,6 @@ int upload(Layout&& L, int device, qh_matrix** out) {
     m->A.iperm = reinterpret_cast<const int32_t*>(base + S.iperm);
     m->A.lr = reinterpret_cast<const LowRankDesc*>(base + S.lr);
     m->A.dd = reinterpret_cast<const DenseDesc*>(base + S.dd);
-    m->A.comp_w = base + S.comp_w;
-    m->A.comp_s = reinterpret_cast<const double*>(base + S.comp_s);
     m->A.tasks = reinterpret_cast<const ColTask*>(base + S.tasks);
     m->A.task_rec = reinterpret_cast<const TaskRec*>(base + S.task_rec);
     m->A.qcodes = base + S.qcodes;

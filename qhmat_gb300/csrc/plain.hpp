@@ -19,8 +19,6 @@ struct Arena {
     const int32_t* iperm;  // source index -> clustered position
     const LowRankDesc* lr;
     const DenseDesc* dd;
-    const uint8_t* comp_w;
-    const double* comp_s;
     const ColTask* tasks;
     const TaskRec* task_rec;
     const uint8_t* qcodes;
@@ -61,8 +59,8 @@ namespace {
 
 // Fixed point: x (per rhs column) and u (per row tile) are held as integers
 // X = round(v * 2^(kFixBits - (e - 1022))), |X| <= 2^kFixBits, on one exponent
-// field e; the tensor-core operand is X's eight base-256 limbs (seven unsigned,
-// the top one signed), each an exact f16.
+// field e; the tensor-core operand is X's eight base-256 limbs, all signed (-128 ..
+// 127, the top one -64 .. 64), each an exact f16.
 constexpr int kFixBits = 62;
 
 

@@ -55,8 +55,8 @@ private:
 };
 
 // Run `launch(word)` (returns a QH_* status), wait for the stream and read
-// what the kernels flagged (fail(error, status bits, what failed)).  A call refused for its arguments has launched
-// nothing and returns at once.
+// what the kernels flagged (`fail(error, status bits, what failed)`).  A call
+// refused for its arguments has launched nothing and returns at once.
 template <class Launch, class Fail>
 int checked_call(StatusWords& words, cudaStream_t s, Launch&& launch, Fail&& fail) {
     int* word = nullptr;

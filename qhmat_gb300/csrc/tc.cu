@@ -120,8 +120,8 @@ struct Bars {
     int abort_flag;
 };
 // Step words: column kernel planes | chunks << 4 | last of its item << 8;
-// row kernel info bytes | kSegmentEnd | kItemEnd | 16-row M-tiles << 20 | 64-row
-// tile << 24.  Segment words: accumulators in use | last of its item << 8.
+// row kernel info bytes | kSegmentEnd | kItemEnd | 64-row tile << 24.  Segment
+// words: accumulators in use | last of its item << 8.
 constexpr uint32_t kNoMore = 0xFFFFFFFFu;
 
 __device__ __forceinline__ void init_bars(Bars& S, int b_writers, int drainers) {
@@ -242,6 +242,8 @@ __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[C]) {
 // unsigned multiply-add into 64 bits.  The biases are taken off at the end
 // (join_limbs).
 constexpr unsigned kBias = 0x7F400000u;
+// (128 entries of digits up to 255 times limbs up to 128: adding 0.75 stays in [0.5, 1))
+static_assert(128 * 255 * 128 < 1 << 22, "sums of an accumulator");
 template <int PER>
 __device__ __forceinline__ void add_sums(unsigned long long (&v)[PER][4], const uint32_t (&d)[8 * PER],
                                          unsigned weight) {
@@ -812,7 +814,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         bool ok = true;
         for (StepRuns<true> st(A, n_items, groups, lane); st.valid() && ok; st.next(A)) {
             const int qrows = st.I.shape >> 8, count = st.count();
-            const uint32_t shape = uint32_t(qrows) << 20 | uint32_t((st.I.shape & 255) >> 6) << 24;
+            const uint32_t shape = uint32_t((st.I.shape & 255) >> 6) << 24;
             const bool has = lane < qrows;
             for (int k = 0; k < count; ++k, ++ri) {
                 const int s = ri % kStages;

@@ -242,8 +242,8 @@ class ServingEngine:
 
         self.pool = pool
         self.max_cols = max_cols
-        # the plain form's work grows with the columns it is given, so larger
-        # batches only delay the requests behind them
+        # the plain form's work grows with the columns it is given (in groups
+        # of eight), so larger batches only delay the requests behind them
         self.plain_max_cols = min(plain_max_cols, max_cols)
         self._lib = load_library()
         self._queue: collections.deque = collections.deque()
