@@ -314,7 +314,8 @@ Schedule schedule_units(const std::vector<double>& costs, int warps);
 // are, so the times of both are predicted, in us, from the work lists; the
 // coefficients are least-squares fits to whole applies of 39 matrices (1-D, 2-D
 // and 3-D, 300 .. 100000 unknowns, leaves of 16 .. 128) with 3 .. 33 columns, 8 %
-// and 5 % off in the mean; no choice among them is slower than column by column.  Column by column / tensor memory, us:
+// and 5 % off in the mean; no choice among them is slower than column by column.
+// Column by column / tensor memory, us:
 //                          3 columns   4           5           8           9           16
 //   2048 (1-D, leaf 32)    32 / 25     40 / 25     48 / 28     71 / 28     81 / 35     139 / 35
 //   16384 (1-D, leaf 16)   87 / 134    113 / 137   137 / 161   212 / 169   236 / 300   412 / 321
