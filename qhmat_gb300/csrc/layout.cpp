@@ -953,10 +953,11 @@ Schedule schedule_units(const std::vector<double>& costs, int warps) {
 KernelChoice kernel_choice(const Layout& L, const Schedule& columns, const Schedule& rows, int sms) {
     KernelChoice c;
     // column by column: the warps' mean load, and what the longest has beyond it
-    // (cycles at 2.07 GHz); x and y; B rows written and read
+    // (cycles at 2.07 GHz); x and y; B rows written and read; the launches' share
     const double mean = (columns.total + rows.total) / (16.0 * sms) / 2070.0;
     const double longest = (columns.longest + rows.longest) / 2070.0;
-    c.column = 0.69 * mean + 0.44 * (longest - mean) + 1.7e-4 * double(L.order) + 8.6e-6 * double(L.n_slots);
+    c.column = 1.3 + 0.78 * mean + 0.375 * (longest - mean) + 1.1e-4 * double(L.order) + 3.4e-6 * double(L.n_slots);
+    c.order = double(L.order);
     const auto* items = reinterpret_cast<const TcItem*>(L.arena.data() + L.sec.tc_items);
     const auto* row_items = reinterpret_cast<const TcRowItem*>(L.arena.data() + L.sec.tc_row_items);
     // (a step holds two chunks of at most two planes, or one of more)
@@ -971,10 +972,14 @@ KernelChoice kernel_choice(const Layout& L, const Schedule& columns, const Sched
 bool KernelChoice::tensor(size_t rhs) const {
     if (rhs < 3) return false;
     const double p = double(rhs), groups = double((rhs + 7) / 8);
+    // (the dense diagonal, two columns at a time, has warps of its own in the column
+    // kernel)
+    const double diagonal = dense * double((rhs + 1) & ~size_t(1));
     const double several =
-        rhs <= 4 ? 15.6 + 0.47 * steps + 0.44 * items + 0.82 * row_steps + 0.43 * p * dense
-                 : 16.3 + groups * (0.22 * steps + 1.05 * items + 0.74 * row_steps) + 0.06 * steps + 0.61 * p * dense;
-    return several < 14.0 + p * column;
+        rhs <= 4 ? 14.8 + std::max(0.51 * steps + 0.57 * items, 0.87 * diagonal) + 0.80 * row_steps + 1.1e-4 * p * order
+                 : 16.4 + std::max(groups * (0.48 * steps + 0.89 * items), 0.74 * diagonal) +
+                       0.83 * groups * row_steps + 0.9e-4 * p * order;
+    return 1.01 * several < 9.4 + p * column;  // (in doubt, column by column)
 }
 
 }  // namespace qhg

@@ -312,10 +312,12 @@ Schedule schedule_units(const std::vector<double>& costs, int warps);
 // eight columns, in items of 128 rows and steps with a fixed handshake cost.
 // Both give the same bits.  Where the line lies depends on how full the items
 // are, so the times of both are predicted, in us, from the work lists; the
-// coefficients are least-squares fits to whole applies of 39 matrices (1-D, 2-D
-// and 3-D, 300 .. 100000 unknowns, leaves of 16 .. 128) with 3 .. 33 columns, 8 %
-// and 5 % off in the mean; no choice among them is slower than column by column.
-// Column by column / tensor memory, us:
+// coefficients are least-squares fits to whole applies of 82 matrices (1-D, 2-D
+// and 3-D, 150 .. 100000 unknowns, leaves of 8 .. 128, ranks of 1 .. 33, equal and
+// mixed code widths) with 3 .. 64 columns, 8 % and 6 % off.  Of those 898 applies
+// four would be faster column by column by more than 1.5 % (10 % at most) and 13 on
+// the other kernels (8 % at most); taking the tensor-memory kernels always made 92
+// of them slower, by up to 62 %.  Column by column / tensor memory, us:
 //                          3 columns   4           5           8           9           16
 //   2048 (1-D, leaf 32)    32 / 25     40 / 25     48 / 28     71 / 28     81 / 35     139 / 35
 //   16384 (1-D, leaf 16)   87 / 134    113 / 137   137 / 161   212 / 169   236 / 300   412 / 321
@@ -325,7 +327,7 @@ Schedule schedule_units(const std::vector<double>& costs, int warps);
 //   8192 (3-D, leaf 64)    133 / 82    174 / 82    212 / 91    332 / 92    372 / 158   644 / 163
 // One and two columns never take them (32768 (2-D) x 1: 81 / 155, 9001 x 2: 77 / 105).
 struct KernelChoice {
-    double column = 0;                                      // us a column
+    double column = 0, order = 0;                           // us a column; unknowns
     double steps = 0, items = 0, row_steps = 0, dense = 0;  // per SM, of one pass over the codes
     bool tensor(size_t rhs) const;
 };
